@@ -319,9 +319,11 @@ def _padded(s, slot, nc, ec, tails):
 
 
 def _on_device(s, slots):
-    """Finished batches as their consumer in this process takes them: sizes from the counters, padding by one launch."""
+    """Finished batches as their consumer in this process takes them: sizes from the counters (all of them by one
+    copy), padding by one launch."""
+    words = torch.cat([s.out[k][c] for k in slots for c in ("nc", "ec")]).tolist()
     tails = []
-    out = [_padded(s, k, s.out[k]["nc"].tolist(), s.out[k]["ec"].tolist(), tails) for k in slots]
+    out = [_padded(s, k, words[32 * i:32 * i + 16], words[32 * i + 16:32 * i + 32], tails) for i, k in enumerate(slots)]
     torch._foreach_zero_(tails)
     return out, s.lru
 
