@@ -1,0 +1,31 @@
+"""Kernels at the sizes where their tiling can go wrong: remainders, one row, one past a full tile."""
+import numpy as np
+import pytest
+
+import legion_ibp_b200 as L
+from conftest import small_graph
+from test_gpu_gather import Rig
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("count", [1, 4, 5, 31, 33, 257, 4097])
+@pytest.mark.parametrize("row_bytes", [4, 12, 68, 120, 2052, 2056, 2064])
+def test_flat_gather_row_counts_and_widths(oracle_mod, count, row_bytes):
+    """Rows outside the 16-byte path: 4-, 8- and 16-byte elements, fewer elements than lanes and more, rows per
+    warp from 4 to 32.  The rows are copies, so the comparison is exact."""
+    rng = np.random.default_rng(count * 31 + row_bytes)
+    n = 3000
+    table = rng.integers(0, 256, (n, row_bytes)).astype(np.uint8)
+    ids = rng.integers(0, n, count).astype(np.int32)
+    ids[:: 7] = -1 if count > 7 else ids[:: 7]
+    order = rng.permutation(n).astype(np.int32)
+    rig = Rig(table, ids, count, capacity=n // 2, order=order)
+    got_n, feat, _ = rig.gather(0)
+    assert got_n == count
+    keep = ids >= 0
+    np.testing.assert_array_equal(feat[keep], table[ids[keep]])
+    st = rig.cache.stats()
+    hit = np.isin(ids[keep], order[: n // 2]).sum()
+    assert st["local_hits"] == hit and st["misses"] == keep.sum() - hit
+    rig.close()
