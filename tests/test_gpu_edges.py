@@ -29,3 +29,25 @@ def test_flat_gather_row_counts_and_widths(oracle_mod, count, row_bytes):
     hit = np.isin(ids[keep], order[: n // 2]).sum()
     assert st["local_hits"] == hit and st["misses"] == keep.sum() - hit
     rig.close()
+
+
+@pytest.mark.parametrize("codec", [L.CODEC_INT8, L.CODEC_E4M3])
+@pytest.mark.parametrize("feat_len", [4, 64, 68, 128, 132, 256, 260, 512, 516, 768, 772, 1024, 1028])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_encoder_row_lengths(oracle_mod, codec, feat_len, shift):
+    """Row lengths around what the lanes of a row hold in registers and row counts around the rows that a warp encodes
+    together; shift: source rows that start on 4 instead of 16 bytes.  Bytes equal the host
+    quantiser's."""
+    import torch
+    rng = np.random.default_rng(feat_len + codec)
+    for n in (1, 3, 4, 5, 1000):
+        x = rng.standard_normal((n, feat_len)).astype(np.float32)
+        x[n // 2] = 0.0
+        if n > 4:
+            x[1] = np.where(x[1] > 0, 3e-40, -2e-40)   # the factor of a row of denormals is not finite
+            x[2, 0] = 3e38
+        src = torch.zeros(n * feat_len + 1, device="cuda")
+        src[shift:shift + n * feat_len] = torch.from_numpy(x).reshape(-1).cuda()
+        out = torch.full((n, oracle_mod.quant_row_bytes(feat_len)), 7, dtype=torch.uint8, device="cuda")
+        L.quantize_table(0, codec, src[shift:], n, feat_len, out)
+        np.testing.assert_array_equal(out.cpu().numpy(), oracle_mod.quant_rows(x, codec))
