@@ -281,7 +281,8 @@ int legion_pool_set_batch(LegionPool *p, int32_t iter, int32_t mode, int32_t pip
 int legion_pool_set_rng(LegionPool *p, uint64_t seed, int32_t max_rounds);
 /* First error raised on the device since the last reset (the reference prints and exits,
  * engine/operator_impl.cu:17-25): 0 none, 1 id map full, 2 edge buffer overflow, 3 node buffer
- * overflow, 4 a bulk copy of the gather timed out (the pipe's output is invalid; stop issuing on it);
+ * overflow, 4 a bulk copy of the gather timed out (the pipe's output is invalid; stop issuing on it),
+ * 6 a wait inside the scan of a hop did not end within its limit (the batch ends with the hops before it);
  * 5 a seed id (or a neighbour id stored in the topology) outside [0, n_nodes) was met: such an id is
  * never used as an index, its slot in the batch reads -1 like a slot past the end of the seed list
  * (engine/operator_impl.cu:41-43), and the rest of the batch is complete.  Synchronises `stream`. */

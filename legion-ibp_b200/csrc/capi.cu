@@ -104,8 +104,8 @@ extern "C" int legion_pool_destroy(LegionPool *p)
         cudaFree(p->ids[i]); cudaFree(p->features[i]); cudaFree(p->labels[i]); cudaFree(p->agg_src[i]);
         cudaFree(p->agg_dst[i]); cudaFree(p->node_counter[i]); cudaFree(p->edge_counter[i]);
         cudaFree(p->miss_rows[i]); cudaFree(p->miss_count[i]);
-        cudaFree(p->cache_index[i]); cudaFree(p->src_global[i]); cudaFree(p->map[i]); cudaFree(p->node_rec[i]);
-        cudaFree(p->tile_sum[i]); cudaFree(p->tile_off[i]); cudaFree(p->eslot[i]); cudaFree(p->erank[i]);
+        cudaFree(p->cache_index[i]); cudaFree(p->src_global[i]); cudaFree(p->map[i]);
+        cudaFree(p->edge_rec[i]); cudaFree(p->tile_state[i]);
         cudaFree(p->edge_cnt[i]);
         cudaFree(p->lru_victim[i]); cudaFree(p->ctl[i]); cudaFree(p->bctl[i]);
         cudaFree(p->seed_stage[i]);
@@ -145,11 +145,10 @@ extern "C" int legion_pool_create_ahead(LegionPool **out, int32_t dev_id, int32_
     p->slots = slots;
     // True worst case: every hop samples all nodes found so far (the reference sizes its buffers
     // as B*(1+f1+f1*f2), engine/server.cu:204-216, which is below it).
-    int64_t nodes = batch_size, edges = 0, max_hop_edges = 0, max_inputs = batch_size;
+    int64_t nodes = batch_size, edges = 0, max_hop_edges = 0;
     for (int h = 0; h < hop_num; ++h) {
         p->fanout[h] = fanout[h];
         int64_t e = nodes * fanout[h];
-        if (nodes > max_inputs) max_inputs = nodes;
         if (e > max_hop_edges) max_hop_edges = e;
         edges += e;
         nodes += e;
@@ -163,7 +162,6 @@ extern "C" int legion_pool_create_ahead(LegionPool **out, int32_t dev_id, int32_
     p->max_nodes = nodes;
     p->max_edges = edges;
     p->max_hop_edges = max_hop_edges;
-    p->max_inputs = max_inputs;
     p->feat_rows = nodes;
     p->rng_seed = 0;
     p->max_rounds = 64;
@@ -198,11 +196,6 @@ extern "C" int legion_pool_create_ahead(LegionPool **out, int32_t dev_id, int32_
     const int64_t pad_nodes = round_up(nodes, kTile) + kTile;
     const int64_t pad_edges = round_up(edges > 0 ? edges : 1, kTile) + kTile;
     const int64_t pad_hop_edges = round_up(max_hop_edges > 0 ? max_hop_edges : 1, kTile) + kTile;
-    // node tiles: 1024 inputs each, except the seed hop, which may count in 256-seed tiles
-    int64_t input_tiles = max_inputs / kTile + 2;
-    if (batch_size / 256 + 2 > input_tiles) input_tiles = batch_size / 256 + 2;
-    p->input_tiles = input_tiles;
-    const int64_t tiles = input_tiles + max_hop_edges / kTile + 2;
 
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < pipes && e == cudaSuccess; ++i) {
@@ -225,11 +218,8 @@ extern "C" int legion_pool_create_ahead(LegionPool **out, int32_t dev_id, int32_
         if (e == cudaSuccess) e = dmalloc(&p->cache_index[i], pad_nodes);
         if (e == cudaSuccess) e = dmalloc(&p->src_global[i], pad_edges);
         if (e == cudaSuccess) e = dmalloc(&p->map[i], (int64_t)front + cap);
-        if (e == cudaSuccess) e = dmalloc(&p->node_rec[i], pad_nodes);
-        if (e == cudaSuccess) e = dmalloc(&p->tile_sum[i], tiles);
-        if (e == cudaSuccess) e = dmalloc(&p->tile_off[i], tiles);
-        if (e == cudaSuccess) e = dmalloc(&p->eslot[i], pad_hop_edges);
-        if (e == cudaSuccess) e = dmalloc(&p->erank[i], pad_hop_edges);
+        if (e == cudaSuccess) e = dmalloc(&p->edge_rec[i], pad_hop_edges);
+        if (e == cudaSuccess) e = dmalloc(&p->tile_state[i], pad_hop_edges / kScanThreads);
         if (e == cudaSuccess) e = dmalloc(&p->edge_cnt[i], (hop_num > 0 ? hop_num : 1) * pad_nodes);
         if (e == cudaSuccess) e = dmalloc(&p->lru_victim[i], pad_nodes);
         if (e == cudaSuccess) e = dmalloc(&p->ctl[i], CTL_WORDS);
@@ -241,7 +231,6 @@ extern "C" int legion_pool_create_ahead(LegionPool **out, int32_t dev_id, int32_
             e = cudaMemcpy(p->ctl[i] + CTL_BACK_DIRTY, &one, sizeof(one), cudaMemcpyHostToDevice);
         }
         if (e == cudaSuccess) e = cudaMemset(p->bctl[i], 0, sizeof(BatchCtl));
-        if (e == cudaSuccess) e = cudaMemset(p->eslot[i], 0, sizeof(int32_t) * pad_hop_edges);
         // seeds and labels of a host-provided batch: one allocation, so that one copy brings both in
         if (e == cudaSuccess) e = dmalloc(&p->seed_stage[i], 2 * (int64_t)batch_size);
         if (e == cudaSuccess) p->label_stage[i] = p->seed_stage[i] + batch_size;
@@ -327,7 +316,8 @@ extern "C" int legion_pool_set_rng(LegionPool *p, uint64_t seed, int32_t max_rou
 }
 
 // First error raised by a kernel of this pool since the last reset (0 = none): 1 id map full,
-// 2 edge buffer overflow, 3 node buffer overflow, 4 bulk copy timed out (these stop the batch);
+// 2 edge buffer overflow, 3 node buffer overflow, 4 bulk copy timed out, 6 a wait of the hop's scan timed out (these
+// stop the batch);
 // 5 a seed or neighbour id outside [0, n_nodes) was met: it was skipped without being read, the
 // rest of the batch is complete.  Synchronises the stream.
 extern "C" int legion_pool_device_error(LegionPool *p, void *stream, int32_t *err, int32_t reset)

@@ -35,12 +35,12 @@ void set_error(const char *fmt, ...);
 #define LG_LAUNCH_CHECK() LG_CUDA(cudaGetLastError())
 
 // ---- device-side batch state --------------------------------------------------------------
-// Tile = number of items (nodes or edges) one CTA scans at a time.
+// Tile = number of entries one CTA scans at a time (256 in small hops).
 constexpr int kTile = 1024;
-constexpr int kScanThreads = 256;  // kTile / 4 items per thread
+constexpr int kScanThreads = 256;
 
 // Values stored in the batch-local id map while a hop is in flight: a node that is new in
-// this hop carries kNewBase + (index of the first edge that reached it) until it gets its
+// this hop carries kNewBase + (number of the first entry that reached it) until it gets its
 // local id.  Local ids stay below kNewBase.
 constexpr int32_t kNewBase = 0x40000000;
 // op id of the runner's single lookup + gather over every node of a batch
@@ -54,29 +54,24 @@ enum Ctl {
     CTL_E_TOTAL = 1,   // edges of the hops already finished
     CTL_E_HOP = 2,     // edges of the hop in flight
     CTL_C_HOP = 3,     // new nodes of the hop in flight
-    CTL_TICKET_A = 4,  // "last CTA done" tickets, one per kernel that needs one
-    CTL_TICKET_B = 5,
-    CTL_TICKET_C = 6,
+    CTL_TICKET_A = 4,  // next tile of the scan over the hop's entries
+    CTL_TICKET_C = 6,  // "last CTA done" tickets, one per kernel that needs one
     CTL_ERROR = 7,     // first error raised by a kernel (0 = none)
     CTL_MISS_COUNT = 8,
     CTL_BACK_DIRTY = 9,  // the back region of the id map holds entries (kept across batches until it is cleared)
     CTL_TICKET_D = 10,
     CTL_BAD_IDS = 11,   // sticky: an id outside [0, n_nodes) was met and skipped (reported as DERR_BAD_ID; the batch goes on)
+    CTL_SEEDS_IN = 5,  // the seeds have entered the id map (with the batch's first hop)
+    CTL_LATE_ERROR = 12, // raised inside the scan of a hop; becomes CTL_ERROR when the scan is over
     CTL_WORDS = 16
 };
 
 enum DeviceError { DERR_NONE = 0, DERR_MAP_FULL = 1, DERR_EDGE_OVERFLOW = 2, DERR_NODE_OVERFLOW = 3,
                    DERR_BULK_TIMEOUT = 4,  // a bulk copy of the gather did not complete within its wait limit
-                   DERR_BAD_ID = 5 };      // a node id outside [0, n_nodes) reached the path; it was skipped, not read
+                   DERR_BAD_ID = 5,        // a node id outside [0, n_nodes) reached the path; it was skipped, not read
+                   DERR_SCAN_TIMEOUT = 6 };  // a wait inside the scan of a hop did not end within its limit
 
-struct NodeRec {  // per input node of a hop, written by the count kernel
-    int64_t start;  // first CSR position of the adjacency list
-    int32_t loff;   // exclusive prefix of min(deg, fanout) inside the node's tile
-    int32_t deg;
-};
-static_assert(sizeof(NodeRec) == 16, "NodeRec is read and written as one 16-byte vector");
-
-struct MapSlot {
+struct alignas(8) MapSlot {  // read and claimed as one 8-byte word
     int32_t key;
     int32_t val;
 };
@@ -196,8 +191,7 @@ struct LegionPool {
     int32_t fanout[LEGION_MAX_HOPS];
     int32_t row_bytes_out;
     int32_t pipes;
-    int64_t max_nodes, max_edges, max_hop_edges, max_inputs;
-    int64_t input_tiles;  // entries of tile_sum / tile_off reserved for the counting kernels (edge tiles follow)
+    int64_t max_nodes, max_edges, max_hop_edges;
     int64_t feat_rows;
     // Hand-off buffers, `slots` sets: what a consumer reads (the seven buffers that are published to trainers).
     // With slots == pipes they ARE the pipes' own output buffers below.  With fewer slots than pipes
@@ -222,9 +216,8 @@ struct LegionPool {
     legion::MapSlot *map[LEGION_MAX_PIPES];      // batch-local id map
     uint32_t map_mask;        // back region of the id map: slots - 1
     uint32_t map_front_mask;  // front region: slots - 1
-    legion::NodeRec *node_rec[LEGION_MAX_PIPES];
-    int32_t *tile_sum[LEGION_MAX_PIPES], *tile_off[LEGION_MAX_PIPES];
-    int32_t *eslot[LEGION_MAX_PIPES], *erank[LEGION_MAX_PIPES];
+    int2 *edge_rec[LEGION_MAX_PIPES];            // entries of the hop in flight: (neighbour id, map slot or -1)
+    uint32_t *tile_state[LEGION_MAX_PIPES];      // counts of the tiles of the hop's entries
     uint8_t *edge_cnt[LEGION_MAX_PIPES];         // edges sampled for every destination, hop after hop (one byte each)
     int64_t *lru_victim[LEGION_MAX_PIPES];       // per node: way chosen for insertion, or -1
     int2 *miss_rows[LEGION_MAX_PIPES];           // (row, node id) to fetch from the host table
@@ -249,12 +242,12 @@ namespace legion {
 // kernel launchers (defined in sample.cu / gather.cu / cache.cu)
 extern int g_pdl;
 extern int g_map_front_shift;
-int launch_batch_generate(cudaStream_t s, LegionPool *p, const BatchCtl &ctl, bool defer_seeds = false);
+int launch_batch_generate(cudaStream_t s, LegionPool *p, const BatchCtl &ctl);
 BatchCtl make_batch_ctl(const LegionPool *p, const LegionCache *c, const int32_t *all_ids, const int32_t *all_labels,
                         int32_t total_cap, int64_t first, int32_t size, int64_t n_nodes);
-const void *map_clear_kernel_address();
+const void *batch_start_kernel_address();
 int launch_sample_hop(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop,
-                      int32_t op_id, bool seeds_pending = false);
+                      int32_t op_id);
 int launch_gather(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op_id);
 int launch_publish(cudaStream_t s, LegionPool *p);
 int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op_id);

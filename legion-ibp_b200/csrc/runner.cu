@@ -44,10 +44,10 @@ struct PipeGraph {
     // argument storage of the first kernel (kept alive for cudaGraphExecKernelNodeSetParams)
     uint4 *a_slots;
     int64_t a_pairs, a_back_pairs;
-    int32_t *a_ctl, *a_nc, *a_ec;
+    int32_t *a_ctl, *a_nc, *a_ec, *a_ids, *a_labels;
     legion::BatchCtl *a_bctl;
     legion::BatchCtl a_value;
-    void *args[8];
+    void *args[10];
     bool valid;
     bool launched;  // since the last sync
 };
@@ -303,11 +303,9 @@ static int issue_gather(LegionRunner *r, cudaStream_t s)
 static int issue_sampling(LegionRunner *r, const BatchCtl &v, cudaStream_t s)
 {
     LegionPool *p = r->pool;
-    // with at least one hop, the first hop's counting kernel also takes the seed slice
-    const bool defer = p->hop_num > 0;
-    int rc = launch_batch_generate(s, p, v, defer);
+    int rc = launch_batch_generate(s, p, v);
     for (int h = 0; h < p->hop_num && rc == LEGION_OK; ++h)
-        rc = launch_sample_hop(s, p, r->graph, p->fanout[h], h, LEGION_INTRABATCH_CON * (h + 1), defer && h == 0);
+        rc = launch_sample_hop(s, p, r->graph, p->fanout[h], h, LEGION_INTRABATCH_CON * (h + 1));
     return rc;
 }
 
@@ -361,7 +359,7 @@ static int capture_pipe(LegionRunner *r, int pipe, const BatchCtl &v)
         if (t != cudaGraphNodeTypeKernel) continue;
         cudaKernelNodeParams kp;
         LG_CUDA(cudaGraphKernelNodeGetParams(nodes[i], &kp));
-        if (kp.func == map_clear_kernel_address()) {
+        if (kp.func == batch_start_kernel_address()) {
             g.ctl_node = nodes[i];
             g.ctl_params = kp;
             g.a_slots = *(uint4 **)kp.kernelParams[0];
@@ -372,6 +370,8 @@ static int capture_pipe(LegionRunner *r, int pipe, const BatchCtl &v)
             g.a_bctl = *(BatchCtl **)kp.kernelParams[5];
             g.a_value = v;
             g.a_back_pairs = *(int64_t *)kp.kernelParams[7];
+            g.a_ids = *(int32_t **)kp.kernelParams[8];
+            g.a_labels = *(int32_t **)kp.kernelParams[9];
             found = true;
         }
     }
@@ -382,6 +382,7 @@ static int capture_pipe(LegionRunner *r, int pipe, const BatchCtl &v)
     }
     g.args[0] = &g.a_slots; g.args[1] = &g.a_pairs; g.args[2] = &g.a_ctl; g.args[3] = &g.a_nc;
     g.args[4] = &g.a_ec; g.args[5] = &g.a_bctl; g.args[6] = &g.a_value; g.args[7] = &g.a_back_pairs;
+    g.args[8] = &g.a_ids; g.args[9] = &g.a_labels;
     g.ctl_params.kernelParams = g.args;
     g.ctl_params.extra = nullptr;
     LG_CUDA(cudaGraphInstantiate(&g.exec, graph, 0));

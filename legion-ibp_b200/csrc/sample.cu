@@ -1,15 +1,14 @@
 // Seed batch generation, neighbour sampling, per-hop dedup and relabel.
 //
-// One hop is four launches on one stream, with every size kept on the device:
-//   hop_count   : per input node degree, CSR start and its edge offset inside a 1024-node tile;
-//                 the last CTA to finish turns the tile sums into tile offsets (no host sync);
-//                 over the seeds it can also take the seed slice itself (batch_generate's work)
-//   hop_sample  : one warp per input node draws the neighbours (Philox4x32-10 counter RNG),
-//                 writes the edges at their final positions and enters every neighbour into the
-//                 batch-local id map with atomicMin(first edge index)
-//   hop_flag    : marks the edge that reached a new node first, ranks the marks per tile
-//   hop_finish  : gives new nodes their local ids in order of first appearance and writes the
-//                 local source id of every edge; the last CTA advances the counters
+// A batch is one launch that empties the id map and takes the seed slice, then two launches per hop on one
+// stream, with every size kept on the device:
+//   hop_sample  : G lanes per input node read its CSR range, draw the neighbours (Philox4x32-10 counter RNG)
+//                 and enter every neighbour into the batch-local id map with the minimum of its entry
+//                 numbers (input * fanout + slot: the order of the edges, without knowing how many edges the
+//                 inputs before it have)
+//   hop_finish  : one scan over the entries that counts edges and new nodes together; edges leave at their
+//                 final positions, new nodes get their local ids in order of first appearance, every edge
+//                 gets the local id of its source; the last CTA advances the counters
 // The edge order (input after input, slot after slot) and the node order (first appearance in
 // that edge order) do not depend on scheduling, so a host replay reproduces them bit for bit.
 //
@@ -39,8 +38,26 @@ __device__ __forceinline__ uint32_t mix32(uint32_t h)
     return h;
 }
 
-// Enters `key` and lowers its value to `cand`; returns the slot.  Keys never change once
-// written during a batch, so a stale read can only show "empty", which the CAS then corrects.
+// One probe of map slot `m` for `key`.  True: the slot is the key's, and its value is at most `cand`.
+// A slot is read and claimed as one 8-byte word, key and value together: a key that is met for the first time
+// costs one load and one compare-and-swap, a key whose value is already below `cand` (a seed, a node of an
+// earlier hop, a hub that other inputs have reached) one load.  Values only fall and keys never change once
+// written, so a stale read can only lead to an atomic that changes nothing.
+__device__ __forceinline__ bool map_claim(MapSlot *m, int32_t key, int32_t cand)
+{
+    const unsigned long long empty = ((unsigned long long)(uint32_t)kEmptyVal << 32) | (uint32_t)kEmptyKey;
+    unsigned long long w = __ldcg(reinterpret_cast<const unsigned long long *>(m));
+    if (w == empty) {
+        w = atomicCAS(reinterpret_cast<unsigned long long *>(m), empty,
+                      ((unsigned long long)(uint32_t)cand << 32) | (uint32_t)key);
+        if (w == empty) return true;
+    }
+    if ((int32_t)(uint32_t)w != key) return false;
+    if ((int32_t)(w >> 32) > cand) atomicMin(&m->val, cand);
+    return true;
+}
+
+// Enters `key` and lowers its value to `cand`; returns the slot.
 // The front region is tried first (kFrontProbes slots from the key's home slot).  Slots never empty
 // during a batch, so every thread that carries the same key sees the same first usable slot there, or
 // finds all of them taken by other keys and moves on to the back region, like every other thread
@@ -51,30 +68,14 @@ __device__ __forceinline__ int32_t map_insert_min(MapSlot *map, MapDims dims, in
     const uint32_t h = mix32((uint32_t)key);
     uint32_t s = h & dims.front_mask;
     for (int probe = 0; probe < kFrontProbes; ++probe) {
-        int32_t k = __ldcg(&map[s].key);
-        if (k == kEmptyKey) {
-            int32_t old = atomicCAS(&map[s].key, kEmptyKey, key);
-            k = (old == kEmptyKey) ? key : old;
-        }
-        if (k == key) {
-            atomicMin(&map[s].val, cand);
-            return (int32_t)s;
-        }
+        if (map_claim(&map[s], key, cand)) return (int32_t)s;
         s = (s + 1) & dims.front_mask;
     }
     if (ctl[CTL_BACK_DIRTY] == 0) ctl[CTL_BACK_DIRTY] = 1;
     MapSlot *back = map + dims.front_mask + 1;
     s = mix32(h ^ 0x9E3779B9u) & dims.back_mask;
     for (uint32_t probe = 0; probe <= dims.back_mask; ++probe) {
-        int32_t k = __ldcg(&back[s].key);
-        if (k == kEmptyKey) {
-            int32_t old = atomicCAS(&back[s].key, kEmptyKey, key);
-            k = (old == kEmptyKey) ? key : old;
-        }
-        if (k == key) {
-            atomicMin(&back[s].val, cand);
-            return (int32_t)(dims.front_mask + 1 + s);
-        }
+        if (map_claim(&back[s], key, cand)) return (int32_t)(dims.front_mask + 1 + s);
         s = (s + 1) & dims.back_mask;
     }
     atomicCAS(&ctl[CTL_ERROR], DERR_NONE, DERR_MAP_FULL);
@@ -108,33 +109,37 @@ __device__ __forceinline__ uint32_t draw_below(uint32_t input_index, uint32_t la
     return (uint32_t)__umul64hi(r64, (unsigned long long)n);
 }
 
-// m distinct values of [0, n) in lanes 0..m-1 (m <= 32 < n).  All 32 lanes take part; lanes
-// >= m hold a dummy that can never compare equal.  A lane keeps its draw unless a lane that
-// already holds the value, or a lower lane that drew it in the same round, exists.
+// m distinct values of [0, n) in lanes 0..m-1 of every group of G lanes (m <= G, m < n; m, n and the node are the
+// group's own).  All 32 lanes take part; lanes >= m of a group hold a dummy that can never compare equal.  A lane
+// keeps its draw unless a lane of its group that already holds the value, or a lower lane that drew it in the same
+// round, exists.
+template <int G>
 __device__ __forceinline__ uint32_t draw_distinct(int m, uint32_t n, uint32_t input_index, uint32_t hop,
-                                                  uint32_t batch_id, uint32_t k0, uint32_t k1,
-                                                  int max_rounds, int lane)
+                                                  uint32_t batch_id, uint32_t k0, uint32_t k1, int max_rounds, int lane)
 {
-    bool kept = lane >= m;
+    const int sub = lane & (G - 1);
+    const unsigned group = (G == 32 ? kFull : ((1u << (G & 31)) - 1u)) << (lane & ~(G - 1));
+    bool kept = sub >= m;
     uint32_t x = 0x80000000u | (uint32_t)lane;
     for (int r = 0; r < max_rounds; ++r) {
-        unsigned keptmask = __ballot_sync(kFull, kept);
-        if (keptmask == kFull) break;
-        if (!kept) x = draw_below(input_index, (uint32_t)lane, (uint32_t)r, hop, batch_id, k0, k1, n);
-        unsigned peers = __match_any_sync(kFull, x);
+        const unsigned keptmask = __ballot_sync(kFull, kept);
+        if (keptmask == kFull) return x;
+        if (!kept) x = draw_below(input_index, (uint32_t)sub, (uint32_t)r, hop, batch_id, k0, k1, n);
+        const unsigned peers = __match_any_sync(kFull, x) & group;
         if (!kept) kept = ((peers & keptmask) == 0u) && ((__ffs(peers) - 1) == lane);
     }
     // Lanes still without a value after max_rounds take the next free value, in lane order.
     unsigned keptmask = __ballot_sync(kFull, kept);
-    for (int guard = 0; guard < 32 && keptmask != kFull; ++guard) {
-        int l = __ffs(~keptmask) - 1;
+    for (int guard = 0; guard < G && keptmask != kFull; ++guard) {
+        const unsigned open = ~keptmask & group;
+        const int l = open != 0u ? __ffs(open) - 1 : lane;
         uint32_t cand = __shfl_sync(kFull, x, l);
         for (int it = 0; it < 64; ++it) {
-            unsigned clash = __ballot_sync(kFull, kept && lane < m && x == cand);
-            if (!clash) break;
-            cand = (cand + 1u) % n;
+            const unsigned clash = __ballot_sync(kFull, open != 0u && kept && sub < m && x == cand);
+            if (clash == 0u) break;
+            if (clash & group) cand = (cand + 1u) % n;
         }
-        if (lane == l) { x = cand; kept = true; }
+        if (lane == l && open != 0u) { x = cand; kept = true; }
         keptmask = __ballot_sync(kFull, kept);
     }
     return x;
@@ -162,36 +167,6 @@ __device__ __forceinline__ int block_excl_scan(int x, int *total, int *smem)
     __syncthreads();
     *total = tot;
     return wo + incl - x;
-}
-
-// The CTA that takes the last ticket turns tile sums into exclusive tile offsets and
-// returns the grand total through *out_total (valid in thread 0 of that CTA only).
-__device__ __forceinline__ bool last_cta_scan(int32_t *ticket, const int32_t *tile_sum, int32_t *tile_off,
-                                              int n_tiles, int *smem, int *s_flag, int *out_total)
-{
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = atomicAdd(ticket, 1);
-        *s_flag = (t == (int)gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!*s_flag) return false;
-    __threadfence();
-    int running = 0;
-    for (int c0 = 0; c0 < n_tiles; c0 += kScanThreads) {
-        int idx = c0 + threadIdx.x;
-        int x = idx < n_tiles ? __ldcg(&tile_sum[idx]) : 0;
-        int tot;
-        int ex = block_excl_scan(x, &tot, smem);
-        if (idx < n_tiles) tile_off[idx] = running + ex;
-        running += tot;
-    }
-    if (threadIdx.x == 0) {
-        *ticket = 0;
-        *out_total = running;
-    }
-    return true;
 }
 
 // literal restatement of counter_update (operator_impl.cu:58-91), executed by one thread
@@ -222,28 +197,45 @@ __device__ __forceinline__ void counter_update(int32_t *nc, int32_t *ec, int op_
 
 // ---- batch start -----------------------------------------------------------------------------
 
-// First kernel of every batch: empties the id map, zeroes the counters and stores the batch's
-// parameters, the only values of the batch that are passed by value.  The front region of the map is
-// always cleared; the back region only if the last batch on this pipe put anything there.
-__global__ void map_clear_kernel(uint4 *slots2, int64_t n_pairs, int32_t *ctl, int32_t *nc, int32_t *ec,
-                                 BatchCtl *bctl, BatchCtl value, int64_t back_pairs)
+// First kernel of every batch: empties the id map, zeroes the counters, stores the batch's parameters (the only
+// values of the batch that are passed by value) and takes the seed slice with its labels (batch_generate,
+// operator_impl.cu:28-56).  The front region of the map is always cleared; the back region only if the last batch
+// on this pipe put anything there.  The seeds enter the map with the first hop.
+__global__ void batch_start_kernel(uint4 *slots2, int64_t n_pairs, int32_t *ctl, int32_t *nc, int32_t *ec,
+                                   BatchCtl *bctl, BatchCtl value, int64_t back_pairs, int32_t *ids, int32_t *labels)
 {
     __shared__ int s_last;
     const bool back_dirty = ctl[CTL_BACK_DIRTY] != 0;  // final since the end of the last batch's sampling
     if (blockIdx.x == 0 && threadIdx.x == 32) *bctl = value;
+    if (blockIdx.x == 0 && threadIdx.x < 16) {
+        // the error word is sticky; the dirty flag and its ticket are read by every CTA of this kernel
+        if (threadIdx.x != CTL_ERROR && threadIdx.x != CTL_BAD_IDS && threadIdx.x != CTL_BACK_DIRTY && threadIdx.x != CTL_TICKET_D)
+            ctl[threadIdx.x] = threadIdx.x == CTL_N_NODES ? value.size : 0;
+        nc[threadIdx.x] = 0;  // cudaMemsetAsync of both counters, operator_impl.cu:158-159
+        ec[threadIdx.x] = 0;
+        __syncwarp(0xFFFFu);
+        if (threadIdx.x == 0) counter_update(nc, ec, 0, value.size, value.hop_num);
+    }
+    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < value.size; idx += gridDim.x * blockDim.x) {
+        const int64_t pos = value.first + idx;
+        int32_t id = -1, label = -1;
+        if (pos < value.total_cap) {  // operator_impl.cu:41-43
+            id = value.all_ids[pos];
+            label = value.all_labels[pos];
+            if (id >= value.n_nodes) {  // not a node of this graph: skipped like an overrun slot, and reported
+                id = -1;
+                ctl[CTL_BAD_IDS] = 1;
+            }
+        }
+        ids[idx] = id;
+        labels[idx] = label;
+    }
     const uint4 empty = make_uint4((uint32_t)kEmptyKey, (uint32_t)kEmptyVal, (uint32_t)kEmptyKey,
                                    (uint32_t)kEmptyVal);
     const int64_t total = n_pairs + (back_dirty ? back_pairs : 0);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x)
         slots2[i] = empty;
-    if (blockIdx.x == 0 && threadIdx.x < 16) {
-        // the error word is sticky; the dirty flag and its ticket are read by every CTA of this kernel
-        if (threadIdx.x != CTL_ERROR && threadIdx.x != CTL_BAD_IDS && threadIdx.x != CTL_BACK_DIRTY && threadIdx.x != CTL_TICKET_D)
-            ctl[threadIdx.x] = 0;
-        nc[threadIdx.x] = 0;  // cudaMemsetAsync of both counters, operator_impl.cu:158-159
-        ec[threadIdx.x] = 0;
-    }
     // the last CTA to get here lowers the flag: every CTA has read it by then, and nothing enters the
     // map before the next kernel
     __syncthreads();
@@ -258,284 +250,240 @@ __global__ void map_clear_kernel(uint4 *slots2, int64_t n_pairs, int32_t *ctl, i
     }
 }
 
-__global__ void batch_generate_kernel(const BatchCtl *__restrict__ b, int32_t *ids, int32_t *labels, MapSlot *map,
-                                      MapDims mask, int32_t *ctl, int32_t *nc, int32_t *ec)
-{
-    pdl_wait();
-    pdl_trigger();
-    const int32_t *__restrict__ all_ids = b->all_ids;
-    const int32_t *__restrict__ all_labels = b->all_labels;
-    const int32_t total_cap = b->total_cap, size = b->size, hop_num = b->hop_num;
-    const int64_t first = b->first;
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < size) {
-        int64_t pos = first + idx;
-        if (pos >= total_cap) {  // operator_impl.cu:41-43
-            ids[idx] = -1;
-            labels[idx] = -1;
-        } else {
-            int32_t id = all_ids[pos % total_cap];
-            if (id >= b->n_nodes) {  // not a node of this graph: skipped like an overrun slot, and reported
-                id = -1;
-                ctl[CTL_BAD_IDS] = 1;
-            }
-            ids[idx] = id;
-            labels[idx] = all_labels[pos % total_cap];
-            if (id >= 0) map_insert_min(map, mask, id, idx, ctl);
-        }
-    }
-    if (idx == 0) {
-        counter_update(nc, ec, 0, size, hop_num);
-        ctl[CTL_N_NODES] = size;
-        ctl[CTL_E_TOTAL] = 0;
-    }
-}
-
 // ---- one hop -----------------------------------------------------------------------------------
 
-// FIRST: the hop over the seeds also does the work of batch_generate_kernel (seed slice, labels, seeds
-// into the id map, counter words of op 0), which saves one launch per batch.
-template <bool FIRST>
-__global__ void __launch_bounds__(kScanThreads)
-hop_count_kernel(const int64_t *__restrict__ indptr, int32_t *ids, int32_t fanout,
-                 NodeRec *rec, int32_t *tile_sum, int32_t *tile_off, int32_t *ctl, int64_t max_edges,
-                 const BatchCtl *__restrict__ b, int32_t *labels, MapSlot *map, MapDims mask, int32_t *nc, int32_t *ec)
-{
-    pdl_wait();
-    pdl_trigger();
-    // the seeds are few (one batch): one item per thread and 256-node tiles give that launch 4 x the CTAs
-    constexpr int IPT = FIRST ? 1 : 4;
-    constexpr int TILE = kScanThreads * IPT;
-    __shared__ int smem[kScanThreads / 32];
-    __shared__ int s_flag;
-    const int n = FIRST ? b->size : ctl[CTL_N_NODES];
-    const int n_limit = b->n_nodes;
-    const int n_tiles = (n + TILE - 1) / TILE;
-    if (FIRST && blockIdx.x == 0 && threadIdx.x == 0) {
-        counter_update(nc, ec, 0, n, b->hop_num);
-        ctl[CTL_N_NODES] = n;
-        ctl[CTL_E_TOTAL] = 0;
-    }
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const int base = tile * TILE + threadIdx.x * IPT;
-        int32_t v[4];
-        if (FIRST) {
-            const int32_t total_cap = b->total_cap;
-            const int64_t first = b->first;
-#pragma unroll
-            for (int j = 0; j < IPT; ++j) {
-                v[j] = -1;
-                const int idx = base + j;
-                if (idx < n) {
-                    const int64_t pos = first + idx;
-                    int32_t lab = -1;
-                    if (pos < total_cap) {  // operator_impl.cu:41-43
-                        v[j] = b->all_ids[pos % total_cap];
-                        lab = b->all_labels[pos % total_cap];
-                        if (v[j] >= n_limit) {  // not a node of this graph: skipped like an overrun slot, and reported
-                            v[j] = -1;
-                            ctl[CTL_BAD_IDS] = 1;
-                        }
-                    }
-                    ids[idx] = v[j];
-                    labels[idx] = lab;
-                    if (v[j] >= 0 && pos < total_cap) map_insert_min(map, mask, v[j], idx, ctl);
-                }
-            }
-        } else {
-            int4 v4 = *reinterpret_cast<const int4 *>(ids + base);  // ids is padded to a whole tile
-            v[0] = v4.x; v[1] = v4.y; v[2] = v4.z; v[3] = v4.w;
-        }
-        int64_t start[4];
-        int32_t deg[4], cnt[4];
-#pragma unroll
-        for (int j = 0; j < IPT; ++j) {
-            start[j] = 0; deg[j] = 0; cnt[j] = 0;
-            if (base + j < n && v[j] >= 0) {
-                if (v[j] < n_limit) {
-                    int64_t s = indptr[v[j]];
-                    int64_t e = indptr[v[j] + 1];
-                    start[j] = s;
-                    deg[j] = (int32_t)(e - s);
-                    cnt[j] = min(deg[j], fanout);
-                } else {  // a neighbour id that the topology itself got wrong is never followed
-                    ctl[CTL_BAD_IDS] = 1;
-                }
-            }
-        }
-        int tsum = 0;
-#pragma unroll
-        for (int j = 0; j < IPT; ++j) tsum += cnt[j];
-        int total;
-        int ex = block_excl_scan(tsum, &total, smem);
-#pragma unroll
-        for (int j = 0; j < IPT; ++j) {
-            if (base + j < n) {
-                NodeRec r;
-                r.start = start[j];
-                r.loff = ex;
-                r.deg = deg[j];
-                *reinterpret_cast<int4 *>(&rec[base + j]) = *reinterpret_cast<int4 *>(&r);
-            }
-            ex += cnt[j];
-        }
-        if (threadIdx.x == 0) tile_sum[tile] = total;
-    }
-    int grand;
-    if (last_cta_scan(&ctl[CTL_TICKET_A], tile_sum, tile_off, n_tiles, smem, &s_flag, &grand)) {
-        if (threadIdx.x == 0) {
-            ctl[CTL_E_HOP] = grand;
-            const int e_total = FIRST ? 0 : ctl[CTL_E_TOTAL];
-            if ((int64_t)e_total + grand > max_edges) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, DERR_EDGE_OVERFLOW);
-        }
-    }
-}
+// Lanes that share an input node: the fanout, rounded up to 8, 16 or 32.
+static inline int group_lanes(int fanout) { return fanout <= 8 ? 8 : fanout <= 16 ? 16 : 32; }
 
-__global__ void __launch_bounds__(256)
-hop_sample_kernel(const int32_t *__restrict__ indices, const NodeRec *__restrict__ rec,
-                  const int32_t *__restrict__ tile_off, int32_t fanout, uint32_t hop,
-                  const BatchCtl *__restrict__ b, int32_t *src_global, int32_t *agg_dst,
-                  int32_t *eslot, MapSlot *map, MapDims mask, int32_t *ctl, int tile_shift,
-                  const int32_t *nc, uint8_t *edge_cnt)
+// A warp takes a chunk of consecutive input nodes: one coalesced load of their ids and one round of loads of their
+// CSR ranges for all of them, then 32 / G nodes at a time, G lanes each, draw their neighbours.
+// Entry i * fanout + s of `rec` holds (neighbour id, its map slot) of slot s of input i, or slot -1.
+// Bound by latency: neighbour id from HBM, map slot and compare-and-swap in L2, one after the other; small chunks
+// keep every warp of the chip on its own chain.
+// In the batch's first hop the seeds enter the map too, each with its position.
+template <int G>
+__global__ void __launch_bounds__(256, 6)
+hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict__ indices, const int32_t *ids,
+                  int32_t fanout, uint32_t hop, const BatchCtl *__restrict__ b, int2 *rec, MapSlot *map, MapDims mask,
+                  int32_t *ctl, const int32_t *nc, uint8_t *edge_cnt, uint32_t *tile_state, int tile_shift,
+                  int64_t max_entries)
 {
     pdl_wait();
     pdl_trigger();
     if (ctl[CTL_ERROR] != DERR_NONE) return;
+    const int n = ctl[CTL_N_NODES];
+    if ((int64_t)n * fanout > max_entries) {  // a hop out of the pool's order: more inputs than this fanout was sized for
+        if (threadIdx.x == 0) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, DERR_EDGE_OVERFLOW);
+        return;
+    }
+    const uint32_t k = (uint32_t)fanout;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, n_threads = gridDim.x * blockDim.x;
+    // the tiles that hop_finish_kernel is about to scan have not been counted yet
+    for (int t = tid, n_tiles = (n * fanout + (1 << tile_shift) - 1) >> tile_shift; t < n_tiles; t += n_threads) tile_state[t] = 0;
     const uint32_t batch_id = b->global_batch, k0 = b->k0, k1 = b->k1;
     const int max_rounds = b->max_rounds;
-    const int n = ctl[CTL_N_NODES];
-    const int e_base = ctl[CTL_E_TOTAL];
-    const int lane = threadIdx.x & 31;
-    const int n_warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t k = (uint32_t)fanout;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += n_warps) {
-        int4 raw = __ldg(reinterpret_cast<const int4 *>(&rec[i]));
-        NodeRec r = *reinterpret_cast<NodeRec *>(&raw);
-        const uint32_t deg = (uint32_t)r.deg;
-        if (lane == 0) {
-            // this hop's per-destination edge counts start behind those of the hops before it, whose destinations
-            // were the nodes known when each began (node_counter words 9 .. 9 + hop - 1; summed here, by one lane,
-            // rather than held in a register of every thread for the whole kernel)
-            int cnt_at = i;
-            for (uint32_t h = 0; h < hop; ++h) cnt_at += __ldg(&nc[LEGION_INTRABATCH_CON * 3 + h]);
-            edge_cnt[cnt_at] = (uint8_t)min(deg, k);
-        }
-        if (deg == 0) continue;
-        const int eh0 = __ldg(&tile_off[i >> tile_shift]) + r.loff;  // tile of the counting kernel that ran before
-        int out_slot = -1;   // slot of this lane's first edge, second edge in out_slot2
-        int out_slot2 = -1;
-        int64_t pos = 0, pos2 = 0;
-        if (deg <= k) {
-            if ((uint32_t)lane < deg) { out_slot = lane; pos = lane; }
-        } else if (deg >= 2 * k) {
-            uint32_t x = draw_distinct((int)k, deg, (uint32_t)i, hop, batch_id, k0, k1, max_rounds, lane);
-            if ((uint32_t)lane < k) { out_slot = lane; pos = x; }
-        } else {
-            const int m = (int)(deg - k);
-            uint32_t x = draw_distinct(m, deg, (uint32_t)i, hop, batch_id, k0, k1, max_rounds, lane);
-            uint32_t mylo = (lane < m && x < 32u) ? (1u << x) : 0u;
-            uint32_t myhi = (lane < m && x >= 32u) ? (1u << (x - 32u)) : 0u;
-            uint32_t exlo = __reduce_or_sync(kFull, mylo);
-            uint32_t exhi = __reduce_or_sync(kFull, myhi);
-            uint32_t validlo = deg >= 32u ? 0xFFFFFFFFu : ((1u << deg) - 1u);
-            uint32_t validhi = deg <= 32u ? 0u : (deg >= 64u ? 0xFFFFFFFFu : ((1u << (deg - 32u)) - 1u));
-            uint32_t keeplo = ~exlo & validlo;
-            uint32_t keephi = ~exhi & validhi;
-            uint32_t below = (1u << lane) - 1u;
-            if ((keeplo >> lane) & 1u) { out_slot = __popc(keeplo & below); pos = lane; }
-            if ((keephi >> lane) & 1u) { out_slot2 = __popc(keeplo) + __popc(keephi & below); pos2 = lane + 32; }
-        }
-        if (out_slot >= 0) {
-            int32_t u = __ldg(&indices[r.start + pos]);
-            int eh = eh0 + out_slot;
-            src_global[e_base + eh] = u;
-            agg_dst[e_base + eh] = i;
-            eslot[eh] = map_insert_min(map, mask, u, kNewBase + eh, ctl);
-        }
-        if (out_slot2 >= 0) {
-            int32_t u = __ldg(&indices[r.start + pos2]);
-            int eh = eh0 + out_slot2;
-            src_global[e_base + eh] = u;
-            agg_dst[e_base + eh] = i;
-            eslot[eh] = map_insert_min(map, mask, u, kNewBase + eh, ctl);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kScanThreads)
-hop_flag_kernel(const int32_t *__restrict__ eslot, const MapSlot *map, int32_t *erank, int32_t *tile_sum,
-                int32_t *tile_off, int32_t *ctl, int64_t max_nodes)
-{
-    pdl_wait();
-    pdl_trigger();
-    __shared__ int smem[kScanThreads / 32];
-    __shared__ int s_flag;
-    const int n_edges = ctl[CTL_E_HOP];
-    const int n_tiles = (n_edges + kTile - 1) / kTile;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const int base = tile * kTile + threadIdx.x * 4;
-        int4 s4 = *reinterpret_cast<const int4 *>(eslot + base);  // eslot is padded to a whole tile
-        int32_t s[4] = { s4.x, s4.y, s4.z, s4.w };
-        int f[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            f[j] = 0;
-            if (base + j < n_edges) f[j] = (__ldcg(&map[s[j]].val) == kNewBase + base + j) ? 1 : 0;
-        }
-        int total;
-        int ex = block_excl_scan(f[0] + f[1] + f[2] + f[3], &total, smem);
-        int4 out;
-        out.x = f[0] ? ex : -1; ex += f[0];
-        out.y = f[1] ? ex : -1; ex += f[1];
-        out.z = f[2] ? ex : -1; ex += f[2];
-        out.w = f[3] ? ex : -1;
-        *reinterpret_cast<int4 *>(erank + base) = out;  // erank is padded to a whole tile
-        if (threadIdx.x == 0) tile_sum[tile] = total;
-    }
-    int grand;
-    if (last_cta_scan(&ctl[CTL_TICKET_B], tile_sum, tile_off, n_tiles, smem, &s_flag, &grand)) {
-        if (threadIdx.x == 0) {
-            ctl[CTL_C_HOP] = grand;
-            if ((int64_t)ctl[CTL_N_NODES] + grand > max_nodes) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, DERR_NODE_OVERFLOW);
-        }
-    }
-}
-
-// New nodes get their local ids (order of first appearance: rank of the flagged edge) and every edge of
-// the hop is relabelled, in one pass.  The local id of a node whose first edge is fe is
-// n0 + tile_off[fe / tile] + erank[fe], which every edge can compute for itself once the flags are
-// scanned; the map entry is rewritten to that id by the first edge, and an edge that reads the entry
-// after the rewrite finds the same number.  The last CTA advances the counters.
-__global__ void hop_finish_kernel(const int32_t *__restrict__ erank, const int32_t *__restrict__ tile_off,
-                                  const int32_t *__restrict__ eslot, const int32_t *__restrict__ src_global,
-                                  int32_t *ids, MapSlot *map, int32_t *agg_src, int32_t *ctl, int32_t *nc, int32_t *ec,
-                                  int op_id, const BatchCtl *__restrict__ b, int last_hop)
-{
-    pdl_wait();
-    pdl_trigger();
-    __shared__ int s_flag;
-    const int n_edges = ctl[CTL_E_HOP];
-    const int n0 = ctl[CTL_N_NODES];
-    const int e_base = ctl[CTL_E_TOTAL];
-    const int c_hop = ctl[CTL_C_HOP];
-    const bool ok = ctl[CTL_ERROR] == DERR_NONE;
-    if (ok) {
-        for (int eh = blockIdx.x * blockDim.x + threadIdx.x; eh < n_edges; eh += gridDim.x * blockDim.x) {
-            const int slot = eslot[eh];
-            const int r = erank[eh];
-            int local;
-            if (r >= 0) {
-                local = n0 + tile_off[eh >> 10] + r;
-                ids[local] = src_global[e_base + eh];
-                map[slot].val = local;
-            } else {
-                local = __ldcg(&map[slot].val);
-                if (local >= kNewBase) {
-                    const int fe = local - kNewBase;
-                    local = n0 + tile_off[fe >> 10] + erank[fe];
+    const int n_limit = b->n_nodes;
+    const bool seeds_in = ctl[CTL_SEEDS_IN] != 0;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+    const unsigned group = (G == 32 ? kFull : ((1u << (G & 31)) - 1u)) << (lane & ~(G - 1));
+    constexpr int NPW = 32 / G;  // nodes that a warp works on together
+    const int n_warps = n_threads >> 5;
+    int chunk = (n + n_warps - 1) / n_warps;
+    chunk = min(32, (chunk + NPW - 1) / NPW * NPW);
+    // this hop's per-destination edge counts start behind those of the hops before it, whose destinations were the
+    // nodes known when each began (node_counter words 9 .. 9 + hop - 1)
+    int cnt0 = 0;
+    for (uint32_t h = 0; h < hop; ++h) cnt0 += __ldcg(&nc[LEGION_INTRABATCH_CON * 3 + h]);
+    for (int64_t first = (int64_t)(tid >> 5) * chunk; first < n; first += (int64_t)n_warps * chunk) {
+        const int here = min(chunk, n - (int)first);
+        int64_t my_start = 0;
+        int32_t my_deg = 0;
+        if (lane < here) {
+            const int32_t id = __ldcg(&ids[first + lane]);
+            if (id >= 0) {
+                if (id < n_limit) {
+                    my_start = __ldg(&indptr[id]);
+                    my_deg = (int32_t)(__ldg(&indptr[id + 1]) - my_start);
+                } else {  // a neighbour id that the topology itself got wrong is never followed
+                    ctl[CTL_BAD_IDS] = 1;
                 }
             }
-            agg_src[e_base + eh] = local;
+            edge_cnt[cnt0 + first + lane] = (uint8_t)min((uint32_t)my_deg, k);
+            if (!seeds_in && id >= 0) map_insert_min(map, mask, id, (int)first + lane, ctl);
+        }
+        for (int j0 = 0; j0 < here; j0 += NPW) {
+            const int j = j0 + lane / G;
+            const int64_t start = __shfl_sync(kFull, (long long)my_start, j & 31);
+            const uint32_t deg_j = (uint32_t)__shfl_sync(kFull, my_deg, j & 31);
+            const uint32_t deg = j < here ? deg_j : 0u;
+            const uint32_t i = (uint32_t)first + (uint32_t)j;
+            // drawn: deg >= 2k draws the k positions to take, k < deg < 2k the deg - k positions to leave out
+            const bool leave_out = deg > k && deg < 2 * k;
+            const int m = deg <= k ? 0 : leave_out ? (int)(deg - k) : (int)k;
+            const uint32_t x = draw_distinct<G>(m, deg, i, hop, batch_id, k0, k1, max_rounds, lane);
+            int out_slot = -1, out_slot2 = -1;   // slot of this lane's first edge, second edge in out_slot2
+            uint32_t pos = sub, pos2 = sub + G;
+            if (!leave_out) {
+                if ((uint32_t)sub < min(deg, k)) out_slot = sub;
+                if (deg > k) pos = x;
+            }
+            if (__any_sync(kFull, leave_out)) {
+                // positions 0 .. deg - 1 without the drawn ones; deg < 2k <= 2G, so two per lane
+                const bool drawn = leave_out && sub < m;
+                const uint32_t out0 = __reduce_or_sync(group, drawn && x < 32u ? 1u << x : 0u);
+                const uint32_t out1 = G == 32 ? __reduce_or_sync(group, drawn && x >= 32u ? 1u << (x - 32u) : 0u) : 0u;
+                if (leave_out) {
+                    const uint32_t keep0 = ~out0 & (deg >= 32u ? 0xFFFFFFFFu : (1u << deg) - 1u);
+                    if ((keep0 >> sub) & 1u) out_slot = __popc(keep0 & ((1u << sub) - 1u));
+                    if (G == 32) {
+                        const uint32_t keep1 = ~out1 & (deg <= 32u ? 0u : (1u << (deg - 32u)) - 1u);
+                        if ((keep1 >> sub) & 1u) out_slot2 = __popc(keep0) + __popc(keep1 & ((1u << sub) - 1u));
+                    } else {
+                        if ((keep0 >> (sub + (G & 31))) & 1u) out_slot2 = __popc(keep0 & ((1u << (sub + (G & 31))) - 1u));
+                    }
+                }
+            }
+            const int e0 = (int)(i * k);
+            int32_t u = 0, u2 = 0;
+            if (out_slot >= 0) u = __ldg(&indices[start + pos]);
+            if (out_slot2 >= 0) u2 = __ldg(&indices[start + pos2]);
+            if (out_slot >= 0) {
+                const int e = e0 + out_slot;
+                rec[e] = make_int2(u, map_insert_min(map, mask, u, kNewBase + e, ctl));
+            }
+            if (out_slot2 >= 0) {
+                const int e = e0 + out_slot2;
+                rec[e] = make_int2(u2, map_insert_min(map, mask, u2, kNewBase + e, ctl));
+            }
+            if (j < here && (uint32_t)sub >= deg && (uint32_t)sub < k) rec[e0 + sub] = make_int2(-1, -1);
+        }
+    }
+}
+
+constexpr int kScanWaitLimit = 1 << 20;
+constexpr uint32_t kTileCounted = 0x80000000u;
+
+// One pass over the entries of a hop, in tiles of 256 * IPT.  A CTA counts its tile's edges and the entries that
+// reached a node first, publishes both counts, adds up the counts of the tiles before it (each CTA reads them all,
+// one word per tile, so nothing is passed from tile to tile) and places its edges and new nodes.
+// Tiles are handed out in order by a ticket and a CTA publishes its counts before it waits for others, so the
+// lowest unfinished tile never waits: whatever else shares the GPU, every wait ends.  All waits are bounded
+// (DERR_SCAN_TIMEOUT).
+// The local id of a node that another entry reached first is written to its map slot by that entry's CTA, which has
+// an earlier tile, or the same one.
+// Bound by L2 latency: record, map slot, counts, map slot.  IPT 1 where the hop is small (a tile for every SM),
+// 4 where it is large (four map reads of a thread in flight, fewer counts to add up).
+template <int IPT>
+__global__ void __launch_bounds__(kScanThreads)
+hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_state, int32_t *ids, MapSlot *map,
+                  int32_t *src_global, int32_t *agg_src, int32_t *agg_dst, int32_t *ctl, int32_t *nc, int32_t *ec, int op_id,
+                  const BatchCtl *__restrict__ b, int last_hop, int64_t max_nodes, int64_t max_edges)
+{
+    pdl_wait();
+    pdl_trigger();
+    constexpr int TILE = kScanThreads * IPT;
+    __shared__ int smem[kScanThreads / 32];
+    __shared__ int s_edges[kScanThreads / 32], s_new[kScanThreads / 32];
+    __shared__ int s_tile, s_flag;
+    const int n0 = ctl[CTL_N_NODES];
+    const int e_base = ctl[CTL_E_TOTAL];
+    const bool ok = ctl[CTL_ERROR] == DERR_NONE;  // raised before this kernel: nobody raises it while it runs
+    const int total = ok ? n0 * fanout : 0;
+    const int n_tiles = (total + TILE - 1) / TILE;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int next = 0, edges = 0, fresh = 0;  // tiles before `next` hold `edges` edges and `fresh` new nodes
+    while ((int)blockIdx.x < n_tiles) {
+        if (threadIdx.x == 0) s_tile = atomicAdd(&ctl[CTL_TICKET_A], 1);
+        __syncthreads();
+        const int tile = s_tile;
+        if (tile >= n_tiles) break;
+        const int base = tile * TILE + threadIdx.x * IPT;
+        int u[IPT], slot[IPT], val[IPT];
+        if constexpr (IPT == 4) {
+            // rec is padded to whole tiles
+            const int4 *r4 = reinterpret_cast<const int4 *>(rec + base);
+            const int4 r0 = __ldcs(r4), r1 = __ldcs(r4 + 1);
+            u[0] = r0.x; slot[0] = r0.y; u[1] = r0.z; slot[1] = r0.w;
+            u[2] = r1.x; slot[2] = r1.y; u[3] = r1.z; slot[3] = r1.w;
+        } else {
+            const int2 r = __ldcs(rec + base);
+            u[0] = r.x; slot[0] = r.y;
+        }
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+            if (base + j >= total) slot[j] = -1;
+            val[j] = slot[j] >= 0 ? __ldcg(&map[slot[j]].val) : 0;
+        }
+        int count = 0;  // edges in the low half, new nodes in the high half: both at most 1024
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) count += (slot[j] >= 0 ? 1 : 0) + (slot[j] >= 0 && val[j] == kNewBase + base + j ? 1 << 16 : 0);
+        int tile_count;
+        int mine = block_excl_scan(count, &tile_count, smem);
+        if (threadIdx.x == 0) *(volatile uint32_t *)&tile_state[tile] = kTileCounted | (uint32_t)tile_count;
+        int se = 0, sn = 0;
+        bool late = false;
+        for (int q = next + threadIdx.x; q < tile; q += kScanThreads) {
+            uint32_t w = __ldcg(&tile_state[q]);
+            for (int spin = 0; (w & kTileCounted) == 0u && spin < kScanWaitLimit; ++spin) w = *(volatile uint32_t *)&tile_state[q];
+            late |= (w & kTileCounted) == 0u;
+            se += (int)(w & 0xFFFFu);
+            sn += (int)((w & ~kTileCounted) >> 16);
+        }
+        se = __reduce_add_sync(kFull, se);
+        sn = __reduce_add_sync(kFull, sn);
+        if (lane == 0) { s_edges[warp] = se; s_new[warp] = sn; }
+        if (__syncthreads_or(late ? 1 : 0)) {
+            if (threadIdx.x == 0) ctl[CTL_LATE_ERROR] = DERR_SCAN_TIMEOUT;
+            break;
+        }
+#pragma unroll
+        for (int w = 0; w < kScanThreads / 32; ++w) { edges += s_edges[w]; fresh += s_new[w]; }
+        const int tile_edges = tile_count & 0xFFFF, tile_new = tile_count >> 16;
+        // (cannot happen with the buffers that legion_pool_create sizes for this fanout)
+        const bool fits = (int64_t)e_base + edges + tile_edges <= max_edges && (int64_t)n0 + fresh + tile_new <= max_nodes;
+        if (!fits) {
+            if (threadIdx.x == 0)
+                ctl[CTL_LATE_ERROR] = (int64_t)e_base + edges + tile_edges > max_edges ? DERR_EDGE_OVERFLOW : DERR_NODE_OVERFLOW;
+            edges += tile_edges; fresh += tile_new; next = tile + 1;
+            __syncthreads();
+            continue;
+        }
+        int at = e_base + edges + (mine & 0xFFFF);
+        int local = n0 + fresh + (mine >> 16);
+        int dst = base / fanout, in_row = base - dst * fanout;
+        int where[IPT];
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+            where[j] = -1;
+            if (slot[j] >= 0) {
+                src_global[at] = u[j];
+                agg_dst[at] = dst;
+                if (val[j] == kNewBase + base + j) {
+                    ids[local] = u[j];
+                    __stcg(&map[slot[j]].val, local);
+                    val[j] = local++;
+                }
+                if (val[j] < kNewBase) agg_src[at] = val[j];
+                else where[j] = at;  // first reached by another entry of this hop
+                ++at;
+            }
+            if (++in_row == fanout) { in_row = 0; ++dst; }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+            if (where[j] < 0) continue;
+            int v = __ldcg(&map[slot[j]].val);
+            for (int spin = 0; v >= kNewBase && spin < kScanWaitLimit; ++spin) v = *(volatile int32_t *)&map[slot[j]].val;
+            if (v >= kNewBase) ctl[CTL_LATE_ERROR] = DERR_SCAN_TIMEOUT;
+            agg_src[where[j]] = v;
+        }
+        edges += tile_edges;
+        fresh += tile_new;
+        next = tile + 1;
+        if (tile == n_tiles - 1 && threadIdx.x == 0) {
+            ctl[CTL_E_HOP] = edges;
+            ctl[CTL_C_HOP] = fresh;
         }
     }
     __threadfence();
@@ -547,8 +495,11 @@ __global__ void hop_finish_kernel(const int32_t *__restrict__ erank, const int32
     __syncthreads();
     if (s_flag && threadIdx.x == 0) {
         // every other CTA has read ctl by now
-        int c = ok ? c_hop : 0;
-        int e = ok ? n_edges : 0;
+        __threadfence();
+        const int late = __ldcg(&ctl[CTL_LATE_ERROR]);
+        if (late != DERR_NONE) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, late);
+        const int c = ok && late == DERR_NONE ? __ldcg(&ctl[CTL_C_HOP]) : 0;
+        const int e = ok && late == DERR_NONE ? __ldcg(&ctl[CTL_E_HOP]) : 0;
         nc[LEGION_INTRABATCH_CON * 2] += c;  // operator_impl.cu:281
         ec[2] += e;                          // operator_impl.cu:282
         counter_update(nc, ec, op_id, 0, 0);
@@ -556,6 +507,8 @@ __global__ void hop_finish_kernel(const int32_t *__restrict__ erank, const int32
         ctl[CTL_E_TOTAL] = e_base + e;
         ctl[CTL_E_HOP] = 0;
         ctl[CTL_C_HOP] = 0;
+        ctl[CTL_TICKET_A] = 0;
+        ctl[CTL_SEEDS_IN] = 1;
         ctl[CTL_TICKET_C] = 0;
     }
     // After the last hop both counter arrays also go to page-locked host memory (one posted store per thread of
@@ -609,7 +562,7 @@ static inline int grid_for(int64_t items, int per_cta, int cap)
     return (int)g;
 }
 
-const void *map_clear_kernel_address() { return (const void *)map_clear_kernel; }
+const void *batch_start_kernel_address() { return (const void *)batch_start_kernel; }
 
 BatchCtl make_batch_ctl(const LegionPool *p, const LegionCache *c, const int32_t *all_ids, const int32_t *all_labels,
                         int32_t total_cap, int64_t first, int32_t size, int64_t n_nodes)
@@ -634,58 +587,57 @@ BatchCtl make_batch_ctl(const LegionPool *p, const LegionCache *c, const int32_t
     return v;
 }
 
-// defer_seeds: only the first kernel (map, counters, batch parameters) is issued; the seed slice is then
-// taken by the first hop (launch_sample_hop with seeds_pending), one launch fewer per batch.
-int launch_batch_generate(cudaStream_t s, LegionPool *p, const BatchCtl &v, bool defer_seeds)
+int launch_batch_generate(cudaStream_t s, LegionPool *p, const BatchCtl &v)
 {
     const int pipe = p->pipe;
     const int64_t n_pairs = ((int64_t)p->map_front_mask + 1) / 2;
     const int64_t back_pairs = ((int64_t)p->map_mask + 1) / 2;
-    // sized for the front region; when the back region has to be cleared too, the CTAs loop longer
-    map_clear_kernel<<<grid_for(n_pairs, 256 * 4, p->sm_count * 8), 256, 0, s>>>(
+    // sized for the front region and the seeds; when the back region has to be cleared too, the CTAs loop longer
+    int64_t threads = n_pairs / 4 > p->batch_size ? n_pairs / 4 : p->batch_size;
+    batch_start_kernel<<<grid_for(threads, 256, p->sm_count * 8), 256, 0, s>>>(
         reinterpret_cast<uint4 *>(p->map[pipe]), n_pairs, p->ctl[pipe], p->node_counter[pipe], p->edge_counter[pipe],
-        p->bctl[pipe], v, back_pairs);
+        p->bctl[pipe], v, back_pairs, p->ids[pipe], p->labels[pipe]);
     LG_LAUNCH_CHECK();
-    if (defer_seeds) return LEGION_OK;
-    LG_CUDA(launch_dep(batch_generate_kernel, grid_for(p->batch_size, 256, 1 << 20), 256, s, p->bctl[pipe], p->ids[pipe],
-                       p->labels[pipe], p->map[pipe], MapDims{ p->map_front_mask, p->map_mask }, p->ctl[pipe], p->node_counter[pipe],
-                       p->edge_counter[pipe]));
     return LEGION_OK;
 }
 
-int launch_sample_hop(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop,
-                      int32_t op_id, bool seeds_pending)
+template <int G>
+static cudaError_t launch_hop_sample(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop,
+                                     int64_t inputs, int tile_shift)
 {
     const int pipe = p->pipe;
-    const int cap = p->sm_count * 8;
+    return launch_dep(hop_sample_kernel<G>, grid_for(inputs, 8 * (32 / G), p->sm_count * 6), 256, s, g->indptr, g->indices, p->ids[pipe], fanout,
+                      (uint32_t)hop, p->bctl[pipe], p->edge_rec[pipe], p->map[pipe], MapDims{ p->map_front_mask, p->map_mask },
+                      p->ctl[pipe], p->node_counter[pipe], p->edge_cnt[pipe], p->tile_state[pipe], tile_shift,
+                      p->max_hop_edges);
+}
+
+template <int IPT>
+static cudaError_t launch_hop_finish(cudaStream_t s, LegionPool *p, int32_t fanout, int32_t hop, int32_t op_id, int64_t edges)
+{
+    const int pipe = p->pipe;
+    return launch_dep(hop_finish_kernel<IPT>, grid_for(edges, kScanThreads * IPT, p->sm_count * 8), kScanThreads, s, p->edge_rec[pipe],
+                      fanout, p->tile_state[pipe], p->ids[pipe], p->map[pipe], p->src_global[pipe], p->agg_src[pipe],
+                      p->agg_dst[pipe], p->ctl[pipe], p->node_counter[pipe], p->edge_counter[pipe], op_id, p->bctl[pipe],
+                      hop + 1 == p->hop_num ? 1 : 0, p->max_nodes, p->max_edges);
+}
+
+int launch_sample_hop(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop, int32_t op_id)
+{
     // worst-case sizes of this hop: inputs = all nodes so far, edges = inputs * fanout
     int64_t inputs = p->batch_size;
     for (int h = 0; h < hop; ++h) inputs += inputs * p->fanout[h];
-    int64_t edges = inputs * fanout;
-    int32_t *ctl = p->ctl[pipe];
-    if (seeds_pending) {
-        LG_ARG(hop == 0, "only the first hop can take the seed slice");
-        LG_CUDA(launch_dep(hop_count_kernel<true>, grid_for(inputs, kScanThreads, cap), kScanThreads, s, g->indptr,
-                           p->ids[pipe], fanout, p->node_rec[pipe], p->tile_sum[pipe], p->tile_off[pipe], ctl, p->max_edges,
-                           p->bctl[pipe], p->labels[pipe], p->map[pipe], MapDims{ p->map_front_mask, p->map_mask }, p->node_counter[pipe],
-                           p->edge_counter[pipe]));
-    } else {
-        LG_CUDA(launch_dep(hop_count_kernel<false>, grid_for(inputs, kTile, cap), kScanThreads, s, g->indptr, p->ids[pipe],
-                           fanout, p->node_rec[pipe], p->tile_sum[pipe], p->tile_off[pipe], ctl, p->max_edges, p->bctl[pipe],
-                           p->labels[pipe], p->map[pipe], MapDims{ p->map_front_mask, p->map_mask }, p->node_counter[pipe], p->edge_counter[pipe]));
-    }
-    LG_CUDA(launch_dep(hop_sample_kernel, grid_for(inputs, 8, cap), 256, s, g->indices, p->node_rec[pipe], p->tile_off[pipe],
-                       fanout, (uint32_t)hop, p->bctl[pipe], p->src_global[pipe], p->agg_dst[pipe], p->eslot[pipe],
-                       p->map[pipe], MapDims{ p->map_front_mask, p->map_mask }, ctl, seeds_pending ? 8 : 10,
-                       p->node_counter[pipe], p->edge_cnt[pipe]));
+    const int64_t edges = inputs * fanout;
+    const bool wide = edges > (int64_t)p->sm_count * kTile;  // more entries than one 1024-entry tile per SM
+    const int tile_shift = wide ? 10 : 8;
     static_assert(kScanThreads == 256 && kTile == 1024, "tile shifts above assume 256-thread scans over 1024-item tiles");
-    int32_t *tile_sum2 = p->tile_sum[pipe] + p->input_tiles;
-    int32_t *tile_off2 = p->tile_off[pipe] + p->input_tiles;
-    LG_CUDA(launch_dep(hop_flag_kernel, grid_for(edges, kTile, cap), kScanThreads, s, p->eslot[pipe], p->map[pipe],
-                       p->erank[pipe], tile_sum2, tile_off2, ctl, p->max_nodes));
-    LG_CUDA(launch_dep(hop_finish_kernel, grid_for(edges, 256 * 4, cap), 256, s, p->erank[pipe], tile_off2, p->eslot[pipe],
-                       p->src_global[pipe], p->ids[pipe], p->map[pipe], p->agg_src[pipe], ctl, p->node_counter[pipe],
-                       p->edge_counter[pipe], op_id, p->bctl[pipe], hop + 1 == p->hop_num ? 1 : 0));
+    switch (group_lanes(fanout)) {
+    case 8: LG_CUDA(launch_hop_sample<8>(s, p, g, fanout, hop, inputs, tile_shift)); break;
+    case 16: LG_CUDA(launch_hop_sample<16>(s, p, g, fanout, hop, inputs, tile_shift)); break;
+    default: LG_CUDA(launch_hop_sample<32>(s, p, g, fanout, hop, inputs, tile_shift)); break;
+    }
+    if (wide) LG_CUDA(launch_hop_finish<4>(s, p, fanout, hop, op_id, edges));
+    else LG_CUDA(launch_hop_finish<1>(s, p, fanout, hop, op_id, edges));
     return LEGION_OK;
 }
 

@@ -253,3 +253,38 @@ def test_isolated_nodes_hubs_and_empty_topology(oracle_mod):
             assert e1 == min(fanout[0], 5000) + 3        # the hub's picks + one edge for each of the three leaves
             assert pool.device_error() == 0
         pool.close(); f.close(); g.close()
+
+
+@pytest.mark.parametrize("fanout", [[8], [9, 7], [16, 1], [17, 16], [32, 8], [2, 3, 32]])
+@pytest.mark.parametrize("batch", [1, 31, 257, 1024])
+@pytest.mark.parametrize("max_rounds", [1, 64])
+def test_lane_groups_and_scan_tiles(oracle_mod, fanout, batch, max_rounds):
+    """Fanouts at the edges of the lane groups that share an input (8, 16, 32), degrees on both sides of the fanout and
+    of twice the fanout, batches around the scan's tiles of 256 entries; with one round nearly every draw goes
+    through the lane-ordered fallback."""
+    indptr, indices = small_graph(2500, 30000, 31)
+    rng = np.random.default_rng(batch)
+    train = rng.integers(0, 2500, batch + batch // 2 + 1).astype(np.int32)   # seeds may repeat
+    labels = rng.integers(0, 47, len(train)).astype(np.int32)
+    g, f, pool = _setup(indptr, indices, train, labels, batch, fanout)
+    pool.set_rng(9, max_rounds)
+    for it in range(2):  # the second batch is the ragged tail
+        _run_ops(g, f, pool, batch, it, fanout, global_batch=it)
+        _compare(_fetch(pool), oracle_mod.run_batch(indptr, indices, train, labels, batch, it, fanout, it, 9, max_rounds=max_rounds))
+        assert pool.device_error() == 0
+    pool.close(); f.close(); g.close()
+
+
+def test_large_hop_matches_host_replay(oracle_mod):
+    """A hop of more entries than one 1024-entry tile per SM, and more tiles than CTAs that run at once."""
+    indptr, indices = small_graph(150000, 4000000, 41)
+    rng = np.random.default_rng(3)
+    train = rng.permutation(150000)[:9000].astype(np.int32)
+    labels = np.zeros(len(train), np.int32)
+    g, f, pool = _setup(indptr, indices, train, labels, 9000, [25, 16])
+    pool.set_rng(13, 64)
+    for it in range(2):
+        _run_ops(g, f, pool, 9000, 0, [25, 16], global_batch=it)
+        _compare(_fetch(pool), oracle_mod.run_batch(indptr, indices, train, labels, 9000, 0, [25, 16], it, 13))
+        assert pool.device_error() == 0
+    pool.close(); f.close(); g.close()
