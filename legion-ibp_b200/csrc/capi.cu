@@ -330,9 +330,11 @@ extern "C" int legion_pool_device_error(LegionPool *p, void *stream, int32_t *er
         LG_CUDA(cudaMemcpyAsync(w, p->ctl[i], sizeof(w), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
         LG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
         // an error that stopped the batch comes before "an id was skipped"
-        const int32_t e = w[CTL_ERROR] != 0 ? w[CTL_ERROR] : (w[CTL_BAD_IDS] != 0 ? (int32_t)DERR_BAD_ID : 0);
+        const int32_t stop = w[CTL_ERROR] != 0 ? w[CTL_ERROR] : w[CTL_LATE_ERROR];
+        const int32_t e = stop != 0 ? stop : (w[CTL_BAD_IDS] != 0 ? (int32_t)DERR_BAD_ID : 0);
         if (e != 0 && (*err == 0 || *err == DERR_BAD_ID)) *err = e;
         if (reset && w[CTL_ERROR] != 0) LG_CUDA(cudaMemsetAsync(p->ctl[i] + CTL_ERROR, 0, 4, (cudaStream_t)stream));
+        if (reset && w[CTL_LATE_ERROR] != 0) LG_CUDA(cudaMemsetAsync(p->ctl[i] + CTL_LATE_ERROR, 0, 4, (cudaStream_t)stream));
         if (reset && w[CTL_BAD_IDS] != 0) LG_CUDA(cudaMemsetAsync(p->ctl[i] + CTL_BAD_IDS, 0, 4, (cudaStream_t)stream));
     }
     return LEGION_OK;

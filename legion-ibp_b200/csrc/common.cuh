@@ -50,19 +50,18 @@ constexpr int32_t kEmptyVal = 0x7FFFFFFF;
 
 // ctl[] words (device scratch, one int32 each)
 enum Ctl {
+    // Both by the parity of the hop: hop h reads word h & 1 and leaves its result in the other, so that the CTA
+    // that learns the result may store it while others of the same launch still read.
     CTL_N_NODES = 0,   // nodes known so far (== nc[0] + nc[1])
-    CTL_E_TOTAL = 1,   // edges of the hops already finished
-    CTL_E_HOP = 2,     // edges of the hop in flight
-    CTL_C_HOP = 3,     // new nodes of the hop in flight
-    CTL_TICKET_A = 4,  // next tile of the scan over the hop's entries
-    CTL_TICKET_C = 6,  // "last CTA done" tickets, one per kernel that needs one
+    CTL_E_TOTAL = 2,   // edges of the hops already finished
+    CTL_TILE = 4,      // next tile of the scan over the hop's entries
+    CTL_SEEDS_IN = 5,  // the seeds have entered the id map (with the batch's first hop)
     CTL_ERROR = 7,     // first error raised by a kernel (0 = none)
     CTL_MISS_COUNT = 8,
     CTL_BACK_DIRTY = 9,  // the back region of the id map holds entries (kept across batches until it is cleared)
     CTL_TICKET_D = 10,
     CTL_BAD_IDS = 11,   // sticky: an id outside [0, n_nodes) was met and skipped (reported as DERR_BAD_ID; the batch goes on)
-    CTL_SEEDS_IN = 5,  // the seeds have entered the id map (with the batch's first hop)
-    CTL_LATE_ERROR = 12, // raised inside the scan of a hop; becomes CTL_ERROR when the scan is over
+    CTL_LATE_ERROR = 12, // raised inside the scan of a hop; becomes CTL_ERROR with the next launch
     CTL_WORDS = 16
 };
 

@@ -8,7 +8,7 @@
 //                 inputs before it have)
 //   hop_finish  : one scan over the entries that counts edges and new nodes together; edges leave at their
 //                 final positions, new nodes get their local ids in order of first appearance, every edge
-//                 gets the local id of its source; the last CTA advances the counters
+//                 gets the local id of its source; the CTA of the last tile advances the counters
 // The edge order (input after input, slot after slot) and the node order (first appearance in
 // that edge order) do not depend on scheduling, so a host replay reproduces them bit for bit.
 //
@@ -204,11 +204,22 @@ __device__ __forceinline__ void counter_update(int32_t *nc, int32_t *ec, int op_
 __global__ void batch_start_kernel(uint4 *slots2, int64_t n_pairs, int32_t *ctl, int32_t *nc, int32_t *ec,
                                    BatchCtl *bctl, BatchCtl value, int64_t back_pairs, int32_t *ids, int32_t *labels)
 {
-    __shared__ int s_last;
-    const bool back_dirty = ctl[CTL_BACK_DIRTY] != 0;  // final since the end of the last batch's sampling
+    __shared__ int s_dirty;
+    if (threadIdx.x == 64) {
+        // the CTA that is the last to have read the flag lowers it; nothing enters the map before the next kernel
+        s_dirty = __ldcg(&ctl[CTL_BACK_DIRTY]);  // final since the end of the last batch's sampling
+        __threadfence();
+        if (atomicAdd(&ctl[CTL_TICKET_D], 1) == (int)gridDim.x - 1) {
+            ctl[CTL_BACK_DIRTY] = 0;
+            ctl[CTL_TICKET_D] = 0;
+        }
+    }
     if (blockIdx.x == 0 && threadIdx.x == 32) *bctl = value;
     if (blockIdx.x == 0 && threadIdx.x < 16) {
-        // the error word is sticky; the dirty flag and its ticket are read by every CTA of this kernel
+        // the error words are sticky, and the dirty flag and its ticket belong to the CTAs of this kernel
+        if (threadIdx.x == CTL_LATE_ERROR && ctl[CTL_LATE_ERROR] != DERR_NONE) {
+            if (ctl[CTL_ERROR] == DERR_NONE) ctl[CTL_ERROR] = ctl[CTL_LATE_ERROR];
+        }
         if (threadIdx.x != CTL_ERROR && threadIdx.x != CTL_BAD_IDS && threadIdx.x != CTL_BACK_DIRTY && threadIdx.x != CTL_TICKET_D)
             ctl[threadIdx.x] = threadIdx.x == CTL_N_NODES ? value.size : 0;
         nc[threadIdx.x] = 0;  // cudaMemsetAsync of both counters, operator_impl.cu:158-159
@@ -232,22 +243,11 @@ __global__ void batch_start_kernel(uint4 *slots2, int64_t n_pairs, int32_t *ctl,
     }
     const uint4 empty = make_uint4((uint32_t)kEmptyKey, (uint32_t)kEmptyVal, (uint32_t)kEmptyKey,
                                    (uint32_t)kEmptyVal);
-    const int64_t total = n_pairs + (back_dirty ? back_pairs : 0);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x)
-        slots2[i] = empty;
-    // the last CTA to get here lowers the flag: every CTA has read it by then, and nothing enters the
-    // map before the next kernel
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_pairs; i += step) slots2[i] = empty;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = atomicAdd(&ctl[CTL_TICKET_D], 1);
-        s_last = (t == (int)gridDim.x - 1);
-    }
-    __syncthreads();
-    if (s_last && threadIdx.x == 0) {
-        ctl[CTL_BACK_DIRTY] = 0;
-        ctl[CTL_TICKET_D] = 0;
-    }
+    if (s_dirty == 0) return;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < back_pairs; i += step) slots2[n_pairs + i] = empty;
 }
 
 // ---- one hop -----------------------------------------------------------------------------------
@@ -270,14 +270,19 @@ hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict_
 {
     pdl_wait();
     pdl_trigger();
-    if (ctl[CTL_ERROR] != DERR_NONE) return;
-    const int n = ctl[CTL_N_NODES];
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, n_threads = gridDim.x * blockDim.x;
+    const int late = ctl[CTL_LATE_ERROR];
+    if (tid == 0) {
+        ctl[CTL_TILE] = 0;
+        if (late != DERR_NONE) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, late);
+    }
+    if (ctl[CTL_ERROR] != DERR_NONE || late != DERR_NONE) return;
+    const int n = ctl[CTL_N_NODES + (hop & 1)];
     if ((int64_t)n * fanout > max_entries) {  // a hop out of the pool's order: more inputs than this fanout was sized for
         if (threadIdx.x == 0) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, DERR_EDGE_OVERFLOW);
         return;
     }
     const uint32_t k = (uint32_t)fanout;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, n_threads = gridDim.x * blockDim.x;
     // the tiles that hop_finish_kernel is about to scan have not been counted yet
     for (int t = tid, n_tiles = (n * fanout + (1 << tile_shift) - 1) >> tile_shift; t < n_tiles; t += n_threads) tile_state[t] = 0;
     const uint32_t batch_id = b->global_batch, k0 = b->k0, k1 = b->k1;
@@ -363,18 +368,53 @@ hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict_
 constexpr int kScanWaitLimit = 1 << 20;
 constexpr uint32_t kTileCounted = 0x80000000u;
 
+// The end of a hop that found c nodes and e edges: counter_update for op_id (a multiple of LEGION_INTRABATCH_CON) on
+// both counter arrays, held one word per lane by the warp that calls; with a mirror (the last hop) both arrays also go
+// to page-locked host memory, one posted store per lane: the host learns the sizes of the batch without a copy-engine
+// transfer queued behind other batches' exports.
+__device__ __forceinline__ void advance_counters(int word, int c, int e, int n0, int e_base, int op_id, int32_t *ctl, int32_t *nc,
+                                                 int32_t *ec, int32_t *mirror)
+{
+    constexpr int C = LEGION_INTRABATCH_CON;
+    const int lane = threadIdx.x & 31, h = op_id / C;
+    const int known = __shfl_sync(kFull, word, 0) + __shfl_sync(kFull, word, 1);
+    const int found = __shfl_sync(kFull, word, C * 2) + c;                                  // operator_impl.cu:281
+    const int done = __shfl_sync(kFull, word, 16) + __shfl_sync(kFull, word, 17);
+    const int drawn = __shfl_sync(kFull, word, 18) + e;                                     // operator_impl.cu:282
+    bool changed = true;                                                                    // operator_impl.cu:66-80
+    if (lane == 0) word = known;
+    else if (lane == 1) word = found;
+    else if (lane == C * 2 || lane == 16 + 2) word = 0;
+    else if (lane == C * 2 + 1 || lane == C * 3 + h) word = known + found;
+    else if (lane == 16) word = done;
+    else if (lane == 17 || lane == 16 + C * 3 + h) word = drawn;
+    else if (lane == 16 + C * 4 + h) word = done;
+    else changed = false;
+    if (changed) *(lane < 16 ? nc + lane : ec + (lane - 16)) = word;
+    if (mirror != nullptr) mirror[lane] = word;
+    if (lane == 0) {
+        const int next = h & 1;  // the parity of the hop that follows
+        ctl[CTL_N_NODES + next] = n0 + c;
+        ctl[CTL_E_TOTAL + next] = e_base + e;
+        ctl[CTL_SEEDS_IN] = 1;
+    }
+}
+
 // One pass over the entries of a hop, in tiles of 256 * IPT.  A CTA counts its tile's edges and the entries that
 // reached a node first, publishes both counts, adds up the counts of the tiles before it (each CTA reads them all,
 // one word per tile, so nothing is passed from tile to tile) and places its edges and new nodes.
 // Tiles are handed out in order by a ticket and a CTA publishes its counts before it waits for others, so the
 // lowest unfinished tile never waits: whatever else shares the GPU, every wait ends.  All waits are bounded
 // (DERR_SCAN_TIMEOUT).
+// The CTA of the last tile knows the hop's totals as soon as it has added up the others' and advances the counters
+// there and then: no CTA waits for the end of all others (the two that did, one of them behind a fence over the stores
+// of the whole CTA, were 4 of the 9-11 us that the launch took on two tiles).
 // The local id of a node that another entry reached first is written to its map slot by that entry's CTA, which has
 // an earlier tile, or the same one.
 // Bound by L2 latency: record, map slot, counts, map slot.  IPT 1 where the hop is small (a tile for every SM),
 // 4 where it is large (four map reads of a thread in flight, fewer counts to add up).
 template <int IPT>
-__global__ void __launch_bounds__(kScanThreads)
+__global__ void __launch_bounds__(kScanThreads, 6)
 hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_state, int32_t *ids, MapSlot *map,
                   int32_t *src_global, int32_t *agg_src, int32_t *agg_dst, int32_t *ctl, int32_t *nc, int32_t *ec, int op_id,
                   const BatchCtl *__restrict__ b, int last_hop, int64_t max_nodes, int64_t max_edges)
@@ -384,16 +424,21 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
     constexpr int TILE = kScanThreads * IPT;
     __shared__ int smem[kScanThreads / 32];
     __shared__ int s_edges[kScanThreads / 32], s_new[kScanThreads / 32];
-    __shared__ int s_tile, s_flag;
-    const int n0 = ctl[CTL_N_NODES];
-    const int e_base = ctl[CTL_E_TOTAL];
+    __shared__ int s_tile;
+    if (threadIdx.x == 0) s_tile = atomicAdd(&ctl[CTL_TILE], 1);
+    const int hop = op_id / LEGION_INTRABATCH_CON - 1;
+    const int n0 = ctl[CTL_N_NODES + (hop & 1)];
+    const int e_base = ctl[CTL_E_TOTAL + (hop & 1)];
     const bool ok = ctl[CTL_ERROR] == DERR_NONE;  // raised before this kernel: nobody raises it while it runs
+    // both counter arrays, one word per lane of the first warp (only this kernel changes what it uses of them)
+    const int counter = threadIdx.x < 16 ? nc[threadIdx.x] : threadIdx.x < 32 ? ec[threadIdx.x - 16] : 0;
+    int32_t *const mirror = last_hop ? b->mirror : nullptr;
     const int total = ok ? n0 * fanout : 0;
     const int n_tiles = (total + TILE - 1) / TILE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int next = 0, edges = 0, fresh = 0;  // tiles before `next` hold `edges` edges and `fresh` new nodes
-    while ((int)blockIdx.x < n_tiles) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(&ctl[CTL_TICKET_A], 1);
+    if (n_tiles == 0 && blockIdx.x == 0 && warp == 0) advance_counters(counter, 0, 0, n0, e_base, op_id, ctl, nc, ec, mirror);
+    for (;;) {
         __syncthreads();
         const int tile = s_tile;
         if (tile >= n_tiles) break;
@@ -444,10 +489,10 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
         if (!fits) {
             if (threadIdx.x == 0)
                 ctl[CTL_LATE_ERROR] = (int64_t)e_base + edges + tile_edges > max_edges ? DERR_EDGE_OVERFLOW : DERR_NODE_OVERFLOW;
-            edges += tile_edges; fresh += tile_new; next = tile + 1;
-            __syncthreads();
-            continue;
+            break;
         }
+        if (tile == n_tiles - 1 && warp == 0)
+            advance_counters(counter, fresh + tile_new, edges + tile_edges, n0, e_base, op_id, ctl, nc, ec, mirror);
         int at = e_base + edges + (mine & 0xFFFF);
         int local = n0 + fresh + (mine >> 16);
         int dst = base / fanout, in_row = base - dst * fanout;
@@ -469,7 +514,6 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
             }
             if (++in_row == fanout) { in_row = 0; ++dst; }
         }
-        __syncthreads();
 #pragma unroll
         for (int j = 0; j < IPT; ++j) {
             if (where[j] < 0) continue;
@@ -478,49 +522,11 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
             if (v >= kNewBase) ctl[CTL_LATE_ERROR] = DERR_SCAN_TIMEOUT;
             agg_src[where[j]] = v;
         }
+        if (n_tiles <= (int)gridDim.x) break;  // a tile for every CTA
         edges += tile_edges;
         fresh += tile_new;
         next = tile + 1;
-        if (tile == n_tiles - 1 && threadIdx.x == 0) {
-            ctl[CTL_E_HOP] = edges;
-            ctl[CTL_C_HOP] = fresh;
-        }
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = atomicAdd(&ctl[CTL_TICKET_C], 1);
-        s_flag = (t == (int)gridDim.x - 1);
-    }
-    __syncthreads();
-    if (s_flag && threadIdx.x == 0) {
-        // every other CTA has read ctl by now
-        __threadfence();
-        const int late = __ldcg(&ctl[CTL_LATE_ERROR]);
-        if (late != DERR_NONE) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, late);
-        const int c = ok && late == DERR_NONE ? __ldcg(&ctl[CTL_C_HOP]) : 0;
-        const int e = ok && late == DERR_NONE ? __ldcg(&ctl[CTL_E_HOP]) : 0;
-        nc[LEGION_INTRABATCH_CON * 2] += c;  // operator_impl.cu:281
-        ec[2] += e;                          // operator_impl.cu:282
-        counter_update(nc, ec, op_id, 0, 0);
-        ctl[CTL_N_NODES] = n0 + c;
-        ctl[CTL_E_TOTAL] = e_base + e;
-        ctl[CTL_E_HOP] = 0;
-        ctl[CTL_C_HOP] = 0;
-        ctl[CTL_TICKET_A] = 0;
-        ctl[CTL_SEEDS_IN] = 1;
-        ctl[CTL_TICKET_C] = 0;
-    }
-    // After the last hop both counter arrays also go to page-locked host memory (one posted store per thread of
-    // a warp): the host learns the sizes of the batch without a copy-engine transfer queued behind other batches'
-    // exports.  s_flag is the same for every thread of the CTA.
-    int32_t *host_mirror = last_hop ? b->mirror : nullptr;
-    if (s_flag && host_mirror != nullptr) {
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            host_mirror[threadIdx.x] = threadIdx.x < 16 ? nc[threadIdx.x] : ec[threadIdx.x - 16];
-            __threadfence_system();
-        }
+        if (threadIdx.x == 0) s_tile = atomicAdd(&ctl[CTL_TILE], 1);
     }
 }
 
