@@ -1,6 +1,6 @@
 // Cache lookup fused with the feature gather.
 //
-// One warp owns 32 consecutive rows of the segment: every lane looks up one id (one coalesced id
+// One warp owns up to 32 consecutive rows of the segment: every lane looks up one id (one coalesced id
 // load, one 4-byte table read), turns the answer into a source pointer (this GPU's partition, a
 // peer's partition reached by plain loads over NVLink, or the pinned host table reached by
 // zero-copy loads), and the warp then copies the rows four at a time with 16-byte loads so that
@@ -44,6 +44,8 @@ struct GatherParams {
     const uint8_t *stage_rows;
     const int32_t *stage_pos;
     int32_t stage_base, stage_n;
+    int32_t n_rows;      // rows of a list of the caller's own; -1: the segment of op_id in the counters
+    int32_t rows_per_warp; // fixed by a tunable; 0: chosen by the length of the list
 };
 
 // A missed row that sits in the batch's staging area is served from there like a cached row; `where` 4 keeps
@@ -68,8 +70,13 @@ __device__ __forceinline__ const uint8_t *shfl_ptr(const uint8_t *p, int src)
 // the cumulative counts nc[9+h], which are written once per batch, so that a gather may overlap
 // the sampling of the next hop on another stream.  Block 0 also leaves the (offset, size)
 // snapshot that counter_update writes for a lookup op (operator_impl.cu:85-87).
-__device__ __forceinline__ void segment_of(int32_t *nc, int op_id, int &off, int &n)
+__device__ __forceinline__ void segment_of(int32_t *nc, int op_id, int &off, int &n, int n_rows = -1)
 {
+    if (n_rows >= 0) {
+        off = 0;
+        n = n_rows;
+        return;
+    }
     if (op_id == kOpGatherAll) {
         // every node of the batch in one launch (the runner's choice: one long gather instead of one
         // short one per hop); the snapshot words get the values the last per-hop lookup would leave
@@ -232,42 +239,40 @@ __device__ __forceinline__ int rows_per_warp_for(int n, int n_warps, int least)
 }
 
 // Rows whose size is a multiple of 16 bytes.  VPL = 16-byte vectors per lane per row,
-// R = rows copied together (R * VPL * 512 bytes in flight per warp).  A warp looks 32 ids up, one per
+// R = rows copied together (R * VPL * 512 bytes in flight per warp).  A warp looks up to 32 ids up, one per
 // lane, then copies their rows R at a time; while the first rows of a chunk are in flight it already
 // fetches the id and the table entry of its next chunk, so that only the first lookup of a warp is
-// exposed.
-template <int VPL, int R, int RPW = 32>
+// exposed.  Long lists are bound by HBM; a list that does not give every warp 32 rows, by the chain id -> table ->
+// row and the rounds behind it, so a warp then takes fewer rows, down to 4, and more SMs have some.
+template <int VPL, int R>
 __global__ void __launch_bounds__(256) gather_vec_kernel(GatherParams p)
 {
-    // RPW = rows one warp looks up and copies per chunk (32: one per lane; 16 or 8: the upper lanes idle during
-    // the lookup, but a warp's life is shorter, so the last wave of CTAs costs less)
-    static_assert(RPW == 32 || RPW == 16 || RPW == 8, "rows per warp");
-    static_assert(RPW >= R, "a chunk holds at least one round of rows");
     __shared__ int cta_counts[3];
     if (threadIdx.x < 3) cta_counts[threadIdx.x] = 0;
     __syncthreads();
     int off, n;
-    segment_of(p.nc, p.op_id, off, n);
+    segment_of(p.nc, p.op_id, off, n, p.n_rows);
     const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     const int row_vec = p.row_bytes >> 4;
+    const int rpw = p.rows_per_warp > 0 ? p.rows_per_warp : rows_per_warp_for(n, n_warps, 4);
     int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (blockIdx.x * (blockDim.x >> 5) * RPW >= n) return;  // the whole CTA is past the end
-    int32_t id = (lane < RPW && c * RPW + lane < n) ? __ldg(&p.ids[off + c * RPW + lane]) : -1;
+    if (blockIdx.x * (blockDim.x >> 5) * rpw >= n) return;  // the whole CTA is past the end
+    int32_t id = (lane < rpw && c * rpw + lane < n) ? __ldg(&p.ids[off + c * rpw + lane]) : -1;
     int32_t raw = lookup_raw(p, id);
-    for (; c * RPW < n; c += n_warps) {
-        const int r = c * RPW + lane;
+    for (; c * rpw < n; c += n_warps) {
+        const int r = c * rpw + lane;
         int32_t gidx, host_row;
         int where;
         const uint8_t *src = decode_raw(p, id, raw, gidx, where, host_row);
-        if (lane < RPW && r < n) p.cache_index[off + r] = gidx;
+        if (lane < rpw && r < n) p.cache_index[off + r] = gidx;
         use_staged(p, off + r, where, src);
         if (p.stats != nullptr) count_where(cta_counts, where, lane);
         const MissTicket ticket = miss_begin(p.miss_count, where, src, lane);
-        const int rows_here = min(RPW, n - c * RPW);
-        uint8_t *dst_base = p.dst + (int64_t)(off + c * RPW) * p.row_bytes;
-        const int rn = (c + n_warps) * RPW + lane;
-        id = (lane < RPW && rn < n) ? __ldg(&p.ids[off + rn]) : -1;
+        const int rows_here = min(rpw, n - c * rpw);
+        uint8_t *dst_base = p.dst + (int64_t)(off + c * rpw) * p.row_bytes;
+        const int rn = (c + n_warps) * rpw + lane;
+        id = (lane < rpw && rn < n) ? __ldg(&p.ids[off + rn]) : -1;
         for (int j0 = 0; j0 < rows_here; j0 += R) {
             uint4 v[R][VPL];
             const uint8_t *sp[R];
@@ -424,7 +429,7 @@ __global__ void __launch_bounds__(256) gather_flat_kernel(GatherParams p)
     if (threadIdx.x < 3) cta_counts[threadIdx.x] = 0;
     __syncthreads();
     int off, n;
-    segment_of(p.nc, p.op_id, off, n);
+    segment_of(p.nc, p.op_id, off, n, p.n_rows);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     const int rpw = rows_per_warp_for(n, n_warps, 4);
@@ -872,10 +877,10 @@ __global__ void lru_claim_reset_kernel(const int64_t *__restrict__ victim, const
 
 // ---- launchers ------------------------------------------------------------------------------------------
 
-template <int VPL, int R, int RPW = 32>
+template <int VPL, int R>
 static void launch_vec(int grid, cudaStream_t s, const GatherParams &gp)
 {
-    gather_vec_kernel<VPL, R, RPW><<<grid, 256, 0, s>>>(gp);
+    gather_vec_kernel<VPL, R><<<grid, 256, 0, s>>>(gp);
 }
 // Widest element that divides the row and to which every row of the caches, the staging area and the output is aligned.
 static void launch_flat(int grid, cudaStream_t s, const GatherParams &gp)
@@ -905,18 +910,19 @@ int g_gather_rows = 0; // rows in flight per warp for 512-byte-class rows (0 = d
 
 int g_gather_rpw = 0;  // rows per warp and chunk of the 512-byte-class gather (0 = default); see legion_set_tunable
 
-static int segment_grid(const LegionPool *p, int32_t op_id, int64_t *rows_out, int rows_per_warp = 32, int cps_default = 8)
+// CTAs for the worst-case rows of this segment (the seeds, the new nodes of hop (op_id / 3), or all nodes) at
+// `least` rows per warp, at most `cps` per SM.
+static int segment_grid(const LegionPool *p, int32_t op_id, int64_t *rows_out, int least, int cps)
 {
-    // worst-case rows of this segment: the seeds, or the new nodes of hop (op_id / 3), or all nodes
     int hop = op_id / LEGION_INTRABATCH_CON;  // 0 = seeds
     int64_t rows = p->batch_size;
     int64_t nodes = p->batch_size;
     for (int h = 0; h < hop; ++h) { rows = nodes * p->fanout[h]; nodes += rows; }
     if (op_id == kOpGatherAll) rows = p->max_nodes;
     if (rows_out) *rows_out = rows;
-    int64_t chunks = (rows + rows_per_warp - 1) / rows_per_warp;
+    int64_t chunks = (rows + least - 1) / least;
     int64_t g64 = (chunks + 7) / 8;
-    int cap = p->sm_count * (g_gather_cps > 0 ? g_gather_cps : cps_default) * (32 / rows_per_warp);
+    int64_t cap = (int64_t)p->sm_count * (g_gather_cps > 0 ? g_gather_cps : cps);
     return (int)(g64 < 1 ? 1 : (g64 > cap ? cap : g64));
 }
 
@@ -925,7 +931,7 @@ static int segment_grid(const LegionPool *p, int32_t op_id, int64_t *rows_out, i
 int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op_id)
 {
     const int pipe = p->pipe;
-    const int grid = segment_grid(p, op_id, nullptr);
+    const int grid = segment_grid(p, op_id, nullptr, 32, 8);
     const int row_bytes = p->row_bytes_out;
 
     if (c != nullptr && c->kind == 1) {
@@ -987,6 +993,8 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
     gp.stage_pos = staged ? p->stage_pos : nullptr;
     gp.stage_base = staged ? p->stage_base : 0;
     gp.stage_n = staged ? p->stage_n : 0;
+    gp.n_rows = -1;
+    gp.rows_per_warp = 0;
 
     // the bulk-copy engine has only ever read this GPU's own memory: a clique of more than one GPU keeps the register path
     if (g_gather_engine == 1 && gp.kg == 1 && (c == nullptr || c->codec == LEGION_CODEC_RAW) && row_bytes % 16 == 0 &&
@@ -999,7 +1007,7 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
             attr_set[p->dev_id] = true;
         }
         int64_t rows = 0;
-        segment_grid(p, op_id, &rows);
+        segment_grid(p, op_id, &rows, 32, 8);
         int64_t want = (rows + 32 * kBulkWarps - 1) / (32 * kBulkWarps);
         int per_sm = (int)(200 * 1024 / (smem + 1024));
         if (per_sm < 1) per_sm = 1;
@@ -1020,6 +1028,10 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
     }
     if (row_bytes % 16 == 0 && row_bytes <= 2048) {
         int vpl = (row_bytes / 16 + 31) / 32;
+        const int cps = vpl == 1 && op_id == kOpGatherAll ? 2 : 8;
+        const int vec_grid = g_gather_rpw > 0 && vpl == 1 ? segment_grid(p, op_id, nullptr, g_gather_rpw, cps * 32 / g_gather_rpw)
+                                                          : segment_grid(p, op_id, nullptr, 4, cps);
+        gp.rows_per_warp = vpl == 1 ? g_gather_rpw : 0;
         switch (vpl) {
         case 1:
             // 8 rows (4 KB) in flight per warp measured best on 512-byte rows (2: 0.47-0.55 of the copy
@@ -1028,20 +1040,18 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
             // CTAs per SM (each warp then copies two or three chunks, the next chunk's lookups in flight) it
             // leaves a third of the register file to them: the launch alone is as fast as with eight (46.1 against
             // 45.7 us at 2 x 10^5 rows), the batch is 3% shorter with the whole table cached (70.1 against 72.4 us).
-            if (g_gather_rpw == 16) launch_vec<1, 8, 16>(segment_grid(p, op_id, nullptr, 16), s, gp);
-            else if (g_gather_rpw == 8) launch_vec<1, 8, 8>(segment_grid(p, op_id, nullptr, 8), s, gp);
-            else if (g_gather_rows == 4) launch_vec<1, 4>(grid, s, gp);
-            else if (g_gather_rows == 16) launch_vec<1, 16>(grid, s, gp);
-            else if (g_gather_rows == 2) launch_vec<1, 2>(grid, s, gp);
-            else launch_vec<1, 8>(op_id == kOpGatherAll ? segment_grid(p, op_id, nullptr, 32, 2) : grid, s, gp);
+            if (g_gather_rows == 4) launch_vec<1, 4>(vec_grid, s, gp);
+            else if (g_gather_rows == 16) launch_vec<1, 16>(vec_grid, s, gp);
+            else if (g_gather_rows == 2) launch_vec<1, 2>(vec_grid, s, gp);
+            else launch_vec<1, 8>(vec_grid, s, gp);
             break;
-        case 2: launch_vec<2, 2>(grid, s, gp); break;
-        case 3: launch_vec<3, 2>(grid, s, gp); break;
-        default: launch_vec<4, 2>(grid, s, gp); break;
+        case 2: launch_vec<2, 2>(vec_grid, s, gp); break;
+        case 3: launch_vec<3, 2>(vec_grid, s, gp); break;
+        default: launch_vec<4, 2>(vec_grid, s, gp); break;
         }
     } else {
         LG_ARG(row_bytes % 4 == 0, "row size must be a multiple of 4 bytes");
-        launch_flat(segment_grid(p, op_id, nullptr, 4, 1), s, gp);  // one warp per 4 rows, at most 8 CTAs per SM
+        launch_flat(segment_grid(p, op_id, nullptr, 4, 8), s, gp);
     }
     LG_LAUNCH_CHECK();
     return LEGION_OK;
@@ -1134,24 +1144,9 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[256 + 12 * (siz
 namespace legion {
 
 // byte offsets inside the array
-constexpr size_t kNaCounter = 0;     // 16 int32: the node_counter words the gather kernels read
 constexpr size_t kNaMissCount = 64;  // 8 int32: [0] entries of the miss list, [4] ticket
 constexpr size_t kNaMissRows = 256;  // int2[LEGION_NOALLOC_MAX_ROWS]
 constexpr size_t kNaCacheIndex = 256 + 8 * (size_t)LEGION_NOALLOC_MAX_ROWS;  // int32[LEGION_NOALLOC_MAX_ROWS]
-
-// The array is shared by every call and keeps what the last call left: the words that must start
-// from a known value are rewritten here at the start of each call.
-__global__ void noalloc_setup_kernel(int32_t *nc, int32_t *miss_count, int32_t n_rows)
-{
-    const int t = threadIdx.x;
-    if (t < 16) nc[t] = 0;
-    if (t < 8) miss_count[t] = 0;
-    __syncthreads();
-    if (t == 0) {
-        nc[LEGION_INTRABATCH_CON * 3 - 1] = 0;   // no hops: one segment
-        nc[LEGION_INTRABATCH_CON * 3] = n_rows;  // rows [0, n_rows)
-    }
-}
 
 }  // namespace legion
 
@@ -1193,15 +1188,17 @@ extern "C" int legion_gather_rows_noalloc(void *stream, int32_t dev_id, const in
     LG_CUDA(noalloc_scratch_of(dev_id, &scratch));
     if (n_rows == 0) return LEGION_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    int32_t *nc = reinterpret_cast<int32_t *>(scratch + kNaCounter);
     int32_t *miss_count = reinterpret_cast<int32_t *>(scratch + kNaMissCount);
-    noalloc_setup_kernel<<<1, 32, 0, s>>>(nc, miss_count, (int32_t)n_rows);
-    LG_LAUNCH_CHECK();
+    // The array is shared by every call and keeps what the last call left: a call that may list misses starts from an
+    // empty list.  Without a host table nothing is listed, and the gather is the only launch.
+    if (host_table != nullptr) LG_CUDA(cudaMemsetAsync(miss_count, 0, 32, s));
 
     GatherParams gp;
     gp.ids = ids_dev;
-    gp.nc = nc;
+    gp.nc = nullptr;
     gp.op_id = 1;
+    gp.n_rows = (int32_t)n_rows;
+    gp.rows_per_warp = 0;
     gp.lut = lut_dev;
     gp.capacity = capacity > 0 ? capacity : 1;
     gp.kg = kg;
@@ -1225,8 +1222,8 @@ extern "C" int legion_gather_rows_noalloc(void *stream, int32_t dev_id, const in
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id);
     if (sms <= 0) sms = 148;
-    int64_t g64 = ((n_rows + 31) / 32 + 7) / 8;
-    int grid = (int)(g64 < 1 ? 1 : (g64 > (int64_t)sms * 8 ? (int64_t)sms * 8 : g64));
+    const int64_t g64 = ((n_rows + 3) / 4 + 7) / 8;
+    const int grid = (int)(g64 > (int64_t)sms * 8 ? (int64_t)sms * 8 : g64);
     if (row_bytes % 16 == 0 && row_bytes <= 2048) {
         int vpl = (row_bytes / 16 + 31) / 32;
         switch (vpl) {
@@ -1236,8 +1233,7 @@ extern "C" int legion_gather_rows_noalloc(void *stream, int32_t dev_id, const in
         default: launch_vec<4, 2>(grid, s, gp); break;
         }
     } else {
-        g64 = ((n_rows + 3) / 4 + 7) / 8;
-        launch_flat((int)(g64 > (int64_t)sms * 8 ? (int64_t)sms * 8 : g64), s, gp);
+        launch_flat(grid, s, gp);
     }
     LG_LAUNCH_CHECK();
     if (host_table != nullptr) {

@@ -51,3 +51,31 @@ def test_encoder_row_lengths(oracle_mod, codec, feat_len, shift):
         out = torch.full((n, oracle_mod.quant_row_bytes(feat_len)), 7, dtype=torch.uint8, device="cuda")
         L.quantize_table(0, codec, src[shift:], n, feat_len, out)
         np.testing.assert_array_equal(out.cpu().numpy(), oracle_mod.quant_rows(x, codec))
+
+
+@pytest.mark.parametrize("row_bytes", [16, 512, 528, 1536, 2048])
+@pytest.mark.parametrize("count", [1, 3, 4, 9, 255, 1001, 40000])
+def test_vector_gather_rows_per_warp(oracle_mod, row_bytes, count):
+    """Short lists give a warp 4 rows, long ones up to 32; half of the rows miss.  The allocation-free call as well."""
+    import torch
+    rng = np.random.default_rng(count + row_bytes)
+    n = 5000
+    table = rng.integers(0, 256, (n, row_bytes)).astype(np.uint8)
+    ids = rng.integers(0, n, count).astype(np.int32)
+    order = rng.permutation(n).astype(np.int32)
+    rig = Rig(table, ids, count, capacity=n // 2, order=order)
+    got_n, feat, _ = rig.gather(0)
+    assert got_n == count
+    np.testing.assert_array_equal(feat, table[ids])
+    hit = np.isin(ids, order[: n // 2]).sum()
+    st = rig.cache.stats()
+    assert st["local_hits"] == hit and st["misses"] == count - hit
+    host = torch.from_numpy(table).pin_memory()
+    out = torch.zeros((count, row_bytes), dtype=torch.uint8, device="cuda")
+    for with_host in (False, True, False):
+        out.zero_()
+        L.gather_rows_noalloc(None, 0, torch.from_numpy(ids).cuda(), rig.cache.lut_ptr(), n // 2, 1, 0, [rig.cache.partition()[0]],
+                              host if with_host else None, n, row_bytes, out)
+        want = table[ids] if with_host else np.where(np.isin(ids, order[: n // 2])[:, None], table[ids], 0)
+        np.testing.assert_array_equal(out.cpu().numpy(), want)
+    rig.close()
