@@ -104,6 +104,7 @@ extern "C" int legion_pool_destroy(LegionPool *p)
         cudaFree(p->ids[i]); cudaFree(p->features[i]); cudaFree(p->labels[i]); cudaFree(p->agg_src[i]);
         cudaFree(p->agg_dst[i]); cudaFree(p->node_counter[i]); cudaFree(p->edge_counter[i]);
         cudaFree(p->miss_rows[i]); cudaFree(p->miss_count[i]);
+        cudaFree(p->miss_sorted[i]); cudaFree(p->miss_rank[i]); cudaFree(p->miss_hist[i]);
         cudaFree(p->cache_index[i]); cudaFree(p->src_global[i]); cudaFree(p->map[i]);
         cudaFree(p->edge_rec[i]); cudaFree(p->tile_state[i]);
         cudaFree(p->edge_cnt[i]);
@@ -213,6 +214,10 @@ extern "C" int legion_pool_create_ahead(LegionPool **out, int32_t dev_id, int32_
         if (e == cudaSuccess) e = cudaMemset(p->edge_counter[i], 0, 64);
         if (e == cudaSuccess) e = cudaMemset(p->ids[i], 0xFF, sizeof(int32_t) * pad_nodes);
         if (e == cudaSuccess) e = dmalloc(&p->miss_rows[i], pad_nodes);
+        if (e == cudaSuccess) e = dmalloc(&p->miss_sorted[i], pad_nodes);
+        if (e == cudaSuccess) e = dmalloc(&p->miss_rank[i], pad_nodes);
+        if (e == cudaSuccess) e = dmalloc(&p->miss_hist[i], kMissStretches);
+        if (e == cudaSuccess) e = cudaMemset(p->miss_hist[i], 0, sizeof(int32_t) * kMissStretches);
         if (e == cudaSuccess) e = dmalloc(&p->miss_count[i], 8);
         if (e == cudaSuccess) e = cudaMemset(p->miss_count[i], 0, 32);
         if (e == cudaSuccess) e = dmalloc(&p->cache_index[i], pad_nodes);

@@ -45,6 +45,8 @@ constexpr int kScanThreads = 256;
 constexpr int32_t kNewBase = 0x40000000;
 // op id of the runner's single lookup + gather over every node of a batch
 constexpr int32_t kOpGatherAll = -1;
+// stretches of the host table by which the rows to fetch are ordered
+constexpr int kMissStretches = 4096;
 constexpr int32_t kEmptyKey = -1;
 constexpr int32_t kEmptyVal = 0x7FFFFFFF;
 
@@ -221,6 +223,10 @@ struct LegionPool {
     int64_t *lru_victim[LEGION_MAX_PIPES];       // per node: way chosen for insertion, or -1
     int2 *miss_rows[LEGION_MAX_PIPES];           // (row, node id) to fetch from the host table
     int32_t *miss_count[LEGION_MAX_PIPES];       // [0] entries, [4] ticket
+    int2 *miss_sorted[LEGION_MAX_PIPES];         // the same list by rising table row (miss_order_kernel)
+    int32_t *miss_rank[LEGION_MAX_PIPES];        // per entry: its number among the entries of its stretch of the table
+    int32_t *miss_hist[LEGION_MAX_PIPES];        // entries per stretch; all zero between batches
+    int32_t miss_ordered[LEGION_MAX_PIPES];      // the gathers since the last fetch counted stretches
     int32_t *ctl[LEGION_MAX_PIPES];
     legion::BatchCtl *bctl[LEGION_MAX_PIPES];
     int32_t *seed_stage[LEGION_MAX_PIPES], *label_stage[LEGION_MAX_PIPES];  // device staging for host-provided seeds

@@ -21,6 +21,15 @@ namespace legion {
 
 static constexpr unsigned kFull = 0xFFFFFFFFu;
 
+// List of the rows of a batch whose source is the host table (see miss_begin).
+struct MissSink {
+    int2 *rows;      // (position in ids, host table row)
+    int32_t *count;  // [0] number of entries
+    int32_t *hist;   // entries per stretch of 1 << shift rows, or nullptr
+    int32_t *rank;
+    int32_t shift, n_rows;  // rows of the table
+};
+
 struct GatherParams {
     const int32_t *ids;
     int32_t *nc;  // node_counter of the pipe
@@ -36,8 +45,6 @@ struct GatherParams {
     int32_t row_bytes;   // bytes of one output row
     int32_t slot_bytes;  // bytes of one cached row
     int32_t feature_len; // elements per row (quantised codecs)
-    int2 *miss_rows;     // (position in ids, host table row) of rows whose source is the host table
-    int32_t *miss_count; // [0] number of entries
     int32_t *err;        // device error word of the pipe (sticky), or nullptr
     // rows of uncached seeds that the copy engine staged in device memory for this batch: entry r < stage_n of the
     // id list, when it misses the cache, is row stage_pos[r] - stage_base of stage_rows (nullptr: no staging)
@@ -46,6 +53,7 @@ struct GatherParams {
     int32_t stage_base, stage_n;
     int32_t n_rows;      // rows of a list of the caller's own; -1: the segment of op_id in the counters
     int32_t rows_per_warp; // fixed by a tunable; 0: chosen by the length of the list
+    MissSink miss;
 };
 
 // A missed row that sits in the batch's staging area is served from there like a cached row; `where` 4 keeps
@@ -152,24 +160,35 @@ __device__ __forceinline__ void defer_misses(int2 *miss_rows, int32_t *miss_coun
 // The same in two halves, for a kernel that wants the row copies of the chunk in flight before it needs the
 // list position: the first half counts the chunk's misses, asks for their place in the list (the atomic's answer
 // travels while the rows do) and clears their source pointers; the second half writes the entries.
+// With `hist` an entry is also counted in its stretch of the host table and carries its number there, from which
+// miss_order_kernel makes a list by rising table row.
+__host__ __device__ __forceinline__ int miss_stretch(int32_t host_row, int32_t n_rows, int32_t shift)
+{
+    return (int)((uint32_t)(host_row < n_rows ? host_row : host_row % n_rows) >> shift);
+}
 struct MissTicket {
     unsigned mask;
-    int base;
+    int base, rank;
 };
-__device__ __forceinline__ MissTicket miss_begin(int32_t *miss_count, int where, const uint8_t *&src, int lane)
+__device__ __forceinline__ MissTicket miss_begin(const MissSink &m, int32_t host_row, int where, const uint8_t *&src, int lane)
 {
     MissTicket t;
     t.mask = __ballot_sync(kFull, where == 2);
-    t.base = 0;
-    if (t.mask != 0u && lane == 0) t.base = atomicAdd(&miss_count[0], __popc(t.mask));
-    if (where == 2) src = nullptr;
+    t.base = t.rank = 0;
+    if (t.mask != 0u && lane == 0) t.base = atomicAdd(&m.count[0], __popc(t.mask));
+    if (where == 2) {
+        src = nullptr;
+        if (m.hist != nullptr) t.rank = atomicAdd(&m.hist[miss_stretch(host_row, m.n_rows, m.shift)], 1);
+    }
     return t;
 }
-__device__ __forceinline__ void miss_finish(int2 *miss_rows, const MissTicket &t, int row, int32_t id, int where, int lane)
+__device__ __forceinline__ void miss_finish(const MissSink &m, const MissTicket &t, int row, int32_t host_row, int where, int lane)
 {
     if (t.mask == 0u) return;
-    const int base = __shfl_sync(kFull, t.base, 0);
-    if (where == 2) miss_rows[base + __popc(t.mask & ((1u << lane) - 1u))] = make_int2(row, id);
+    const int at = __shfl_sync(kFull, t.base, 0) + __popc(t.mask & ((1u << lane) - 1u));
+    if (where != 2) return;
+    m.rows[at] = make_int2(row, host_row);
+    if (m.hist != nullptr) m.rank[at] = t.rank;
 }
 
 // Hit / miss counters of a CTA, added to the cache's counters once per CTA (three atomics on three words that
@@ -268,7 +287,7 @@ __global__ void __launch_bounds__(256) gather_vec_kernel(GatherParams p)
         if (lane < rpw && r < n) p.cache_index[off + r] = gidx;
         use_staged(p, off + r, where, src);
         if (p.stats != nullptr) count_where(cta_counts, where, lane);
-        const MissTicket ticket = miss_begin(p.miss_count, where, src, lane);
+        const MissTicket ticket = miss_begin(p.miss, host_row, where, src, lane);
         const int rows_here = min(rpw, n - c * rpw);
         uint8_t *dst_base = p.dst + (int64_t)(off + c * rpw) * p.row_bytes;
         const int rn = (c + n_warps) * rpw + lane;
@@ -302,7 +321,7 @@ __global__ void __launch_bounds__(256) gather_vec_kernel(GatherParams p)
                 }
             }
         }
-        miss_finish(p.miss_rows, ticket, off + r, host_row, where, lane);
+        miss_finish(p.miss, ticket, off + r, host_row, where, lane);
     }
     __syncthreads();
     if (p.stats != nullptr && threadIdx.x < 3 && cta_counts[threadIdx.x] != 0)
@@ -372,7 +391,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32) gather_bulk_kernel(GatherPara
             const uint8_t *src = decode_raw(p, id, raw, gidx, where, host_row);
             if (r < n) p.cache_index[off + r] = gidx;
             add_stats(p.stats, where, lane);
-            defer_misses(p.miss_rows, p.miss_count, off + r, host_row, where, src, lane);
+            defer_misses(p.miss.rows, p.miss.count, off + r, host_row, where, src, lane);
             const int rn = (c + n_warps) * 32 + lane;
             id = (rn < n) ? __ldg(&p.ids[off + rn]) : -1;
             const unsigned hits = __ballot_sync(kFull, src != nullptr);
@@ -446,7 +465,7 @@ __global__ void __launch_bounds__(256) gather_flat_kernel(GatherParams p)
         if (mine) p.cache_index[off + r] = gidx;
         use_staged(p, off + r, where, src);
         if (p.stats != nullptr) count_where(cta_counts, where, lane);
-        const MissTicket ticket = miss_begin(p.miss_count, where, src, lane);
+        const MissTicket ticket = miss_begin(p.miss, host_row, where, src, lane);
         s_src[warp][lane] = src;
         __syncwarp();
         const int total = min(rpw, n - c * rpw) * per_row;
@@ -474,7 +493,7 @@ __global__ void __launch_bounds__(256) gather_flat_kernel(GatherParams p)
             for (int u = 0; u < U; ++u)
                 if (ok[u]) __stcs(&dst[i0 + 32 * u], v[u]);
         }
-        miss_finish(p.miss_rows, ticket, off + r, host_row, where, lane);
+        miss_finish(p.miss, ticket, off + r, host_row, where, lane);
         __syncwarp();
     }
     __syncthreads();
@@ -494,77 +513,76 @@ __device__ __forceinline__ float decode_code(uint8_t b)
 }
 
 template <int CODEC>
+__device__ __forceinline__ float4 decode_word(uint32_t packed, float scale)
+{
+    return make_float4(__fmul_rn(decode_code<CODEC>((uint8_t)(packed)), scale), __fmul_rn(decode_code<CODEC>((uint8_t)(packed >> 8)), scale),
+                       __fmul_rn(decode_code<CODEC>((uint8_t)(packed >> 16)), scale), __fmul_rn(decode_code<CODEC>((uint8_t)(packed >> 24)), scale));
+}
+
+// The same shape as gather_vec_kernel: a lane looks one id up and fetches that row's scale, the warp copies R rows
+// together, V words (128 V codes) of each per lane and step.  Bound by HBM (the fp32 rows written are four fifths of
+// the bytes).  Eight words in flight per lane and, over all nodes of a batch, two CTAs per SM: 16 words and eight CTAs took
+// the registers of the sampling kernels beside it (four batches of 800 seeds, 100 codes a row: 268 us against 234; one
+// row after the other for rows of more than 128 codes was the alternative).
+template <int CODEC, int V, int R>
 __global__ void __launch_bounds__(256) gather_quant_kernel(GatherParams p)
 {
+    __shared__ int cta_counts[3];
+    if (threadIdx.x < 3) cta_counts[threadIdx.x] = 0;
+    __syncthreads();
     int off, n;
     segment_of(p.nc, p.op_id, off, n);
     const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
-    const int f = p.feature_len;
-    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * 32 < n; c += n_warps) {
-        const int r = c * 32 + lane;
-        int32_t id = (r < n) ? __ldg(&p.ids[off + r]) : -1;
+    const int f = p.feature_len, groups = f >> 2;
+    const int rpw = rows_per_warp_for(n, n_warps, 8);
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * rpw < n; c += n_warps) {
+        const int r = c * rpw + lane;
+        const bool mine = lane < rpw && r < n;
+        const int32_t id = mine ? __ldg(&p.ids[off + r]) : -1;
         int32_t gidx, host_row;
         int where;
         const uint8_t *src = resolve(p, id, gidx, where, host_row);
-        if (r < n) p.cache_index[off + r] = gidx;
-        add_stats(p.stats, where, lane);
-        defer_misses(p.miss_rows, p.miss_count, off + r, host_row, where, src, lane);
-        const int rows_here = min(32, n - c * 32);
-        float *dst_base = reinterpret_cast<float *>(p.dst + (int64_t)(off + c * 32) * p.row_bytes);
-        if (f <= 128) {
-            // up to 128 codes per row: one 4-byte word per lane and row, 8 rows in flight per warp
-            constexpr int R = 8;
-            const bool mine = lane < (f >> 2);
-            for (int j0 = 0; j0 < rows_here; j0 += R) {
-                const uint8_t *sp[R];
-                uint32_t packed[R];
-                float scale[R];
+        if (mine) p.cache_index[off + r] = gidx;
+        if (p.stats != nullptr) count_where(cta_counts, where, lane);
+        const MissTicket ticket = miss_begin(p.miss, host_row, where, src, lane);
+        const float my_scale = src != nullptr ? *reinterpret_cast<const float *>(src + f) : 0.0f;  // f is a multiple of 4
+        const int rows_here = min(rpw, n - c * rpw);
+        float *dst_base = reinterpret_cast<float *>(p.dst + (int64_t)(off + c * rpw) * p.row_bytes);
+        for (int j0 = 0; j0 < rows_here; j0 += R) {
+            const uint8_t *sp[R];
+#pragma unroll
+            for (int jj = 0; jj < R; ++jj) {
+                sp[jj] = shfl_ptr(src, (j0 + jj) & 31);   // nullptr: invalid id, or a miss left to the miss kernel
+                if (j0 + jj >= rows_here) sp[jj] = nullptr;
+            }
+            for (int g0 = 0; g0 < groups; g0 += 32 * V) {
+                uint32_t packed[R][V];
 #pragma unroll
                 for (int jj = 0; jj < R; ++jj) {
-                    sp[jj] = shfl_ptr(src, (j0 + jj) & 31);
-                    if (j0 + jj >= rows_here) sp[jj] = nullptr;
-                }
 #pragma unroll
-                for (int jj = 0; jj < R; ++jj) {
-                    if (sp[jj] != nullptr && mine) {
-                        packed[jj] = *reinterpret_cast<const uint32_t *>(sp[jj] + lane * 4);
-                        scale[jj] = *reinterpret_cast<const float *>(sp[jj] + f);
+                    for (int q = 0; q < V; ++q) {
+                        const int g = g0 + lane + 32 * q;
+                        if (sp[jj] != nullptr && g < groups) packed[jj][q] = *reinterpret_cast<const uint32_t *>(sp[jj] + g * 4);
                     }
                 }
 #pragma unroll
                 for (int jj = 0; jj < R; ++jj) {
-                    if (sp[jj] != nullptr && mine) {
-                        float4 o;
-                        o.x = __fmul_rn(decode_code<CODEC>((uint8_t)(packed[jj])), scale[jj]);
-                        o.y = __fmul_rn(decode_code<CODEC>((uint8_t)(packed[jj] >> 8)), scale[jj]);
-                        o.z = __fmul_rn(decode_code<CODEC>((uint8_t)(packed[jj] >> 16)), scale[jj]);
-                        o.w = __fmul_rn(decode_code<CODEC>((uint8_t)(packed[jj] >> 24)), scale[jj]);
-                        __stcs(reinterpret_cast<float4 *>(dst_base + (int64_t)(j0 + jj) * f) + lane, o);
+                    const float scale = __shfl_sync(kFull, my_scale, (j0 + jj) & 31);
+#pragma unroll
+                    for (int q = 0; q < V; ++q) {
+                        const int g = g0 + lane + 32 * q;
+                        if (sp[jj] != nullptr && g < groups)
+                            __stcs(reinterpret_cast<float4 *>(dst_base + (int64_t)(j0 + jj) * f) + g, decode_word<CODEC>(packed[jj][q], scale));
                     }
                 }
             }
-            continue;
         }
-        for (int j = 0; j < rows_here; ++j) {
-            const uint8_t *sp = shfl_ptr(src, j);
-            if (sp == nullptr) continue;  // invalid id, or a miss left to the miss kernel (raw fp32 row)
-            float *drow = dst_base + (int64_t)j * f;
-            {
-                const float scale = *reinterpret_cast<const float *>(sp + f);  // f is a multiple of 4
-                const int groups = f >> 2;
-                for (int g = lane; g < groups; g += 32) {
-                    uint32_t packed = *reinterpret_cast<const uint32_t *>(sp + g * 4);
-                    float4 o;
-                    o.x = __fmul_rn(decode_code<CODEC>((uint8_t)(packed)), scale);
-                    o.y = __fmul_rn(decode_code<CODEC>((uint8_t)(packed >> 8)), scale);
-                    o.z = __fmul_rn(decode_code<CODEC>((uint8_t)(packed >> 16)), scale);
-                    o.w = __fmul_rn(decode_code<CODEC>((uint8_t)(packed >> 24)), scale);
-                    __stcs(reinterpret_cast<float4 *>(drow) + g, o);
-                }
-            }
-        }
+        miss_finish(p.miss, ticket, off + r, host_row, where, lane);
     }
+    __syncthreads();
+    if (p.stats != nullptr && threadIdx.x < 3 && cta_counts[threadIdx.x] != 0)
+        atomicAdd(&p.stats[threadIdx.x], (unsigned long long)cta_counts[threadIdx.x]);
 }
 
 // Rows that miss the cache: one warp copies `R` rows of the miss list at a time from the pinned host
@@ -585,7 +603,44 @@ struct MissParams {
     uint8_t *dst;
     int32_t row_bytes;
     int32_t host_row_bytes;  // bytes of one row of the host table (compressed host tables: codes + scale, padded)
+    int32_t *hist;           // counts of stretches to be zeroed for the next batch, or nullptr
 };
+
+// The miss list by rising table row, up to the order inside a stretch: place of an entry = entries of the stretches
+// before its own + its number there.  Every CTA adds up all the counts for itself.
+// Why: the host link's translations are shared by rows that lie close together and are asked for together.  Measured
+// over a 4 GB table, 512-byte rows: 80,000 random rows 36.0 GB/s, sorted 47.6, by 4096 stretches 46.7, by 256 38.7;
+// 20,000 rows 31.2, sorted 37.0, by 4096 stretches 36.8.
+__global__ void __launch_bounds__(1024)
+miss_order_kernel(const int2 *__restrict__ list, const int32_t *__restrict__ rank, const int32_t *__restrict__ count,
+                  const int32_t *__restrict__ hist, int32_t shift, int32_t n_rows, int2 *out)
+{
+    static_assert(kMissStretches == 4096, "four counts per thread");
+    __shared__ int32_t before[kMissStretches];
+    __shared__ int32_t warp_sum[32];
+    const int n = count[0];
+    if ((int)(blockIdx.x * blockDim.x) >= n) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int4 h = reinterpret_cast<const int4 *>(hist)[threadIdx.x];
+    const int mine = h.x + h.y + h.z + h.w;
+    int incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += t;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    int at = incl - mine + __reduce_add_sync(kFull, lane < warp ? warp_sum[lane] : 0);
+    int4 b;
+    b.x = at; b.y = b.x + h.x; b.z = b.y + h.y; b.w = b.z + h.z;
+    reinterpret_cast<int4 *>(before)[threadIdx.x] = b;
+    __syncthreads();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int2 e = list[i];
+        out[before[miss_stretch(e.y, n_rows, shift)] + rank[i]] = e;
+    }
+}
 
 // The list is complete and consumed: the last CTA to finish empties it for the next batch.
 __device__ __forceinline__ void miss_list_done(const MissParams &p, int *s_last)
@@ -602,12 +657,23 @@ __device__ __forceinline__ void miss_list_done(const MissParams &p, int *s_last)
     }
 }
 
+__device__ __forceinline__ void miss_zero_hist(const MissParams &p)
+{
+    if (p.hist != nullptr && blockIdx.x == 0)
+        for (int t = threadIdx.x; t < kMissStretches; t += blockDim.x) p.hist[t] = 0;
+}
+
 // Host table stored as compressed rows (feature_len one-byte codes + fp32 scale): the fetch moves
 // host_row_bytes per row over the host link instead of 4 * feature_len and decodes into the fp32 output row.
-template <int CODEC, int R>
+// Bound by the requests that the link takes (~380 a microsecond, whatever their size up to 128 bytes): NARROW rows (at most
+// 32 vectors) are read by one 16-byte load per lane, scale included, which is as few requests as the row has 128-byte
+// lines, and the words change lanes on the way to the output row; longer rows load the scale on its own.  Measured,
+// 13,150 rows of 144 bytes: 110 -> 75 us, a batch of 8000 seeds 110 -> 81 us.
+template <int CODEC, int R, bool NARROW>
 __global__ void __launch_bounds__(1024) gather_miss_quant_kernel(MissParams p)
 {
     __shared__ int s_last;
+    miss_zero_hist(p);
     const int n = p.miss_count[0];
     const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
@@ -617,7 +683,6 @@ __global__ void __launch_bounds__(1024) gather_miss_quant_kernel(MissParams p)
     for (int m0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * R; m0 < n; m0 += n_warps * R) {
         const uint8_t *sp[R];
         float *dp[R];
-        float scale[R];
 #pragma unroll
         for (int jj = 0; jj < R; ++jj) {
             sp[jj] = nullptr;
@@ -628,25 +693,41 @@ __global__ void __launch_bounds__(1024) gather_miss_quant_kernel(MissParams p)
                 dp[jj] = reinterpret_cast<float *>(p.dst + (int64_t)e.x * p.row_bytes);
             }
         }
-#pragma unroll
-        for (int jj = 0; jj < R; ++jj)
-            if (sp[jj] != nullptr) scale[jj] = *reinterpret_cast<const float *>(sp[jj] + f);
-        for (int g0 = 0; g0 < groups; g0 += 32) {
-            const int g = g0 + lane;
-            uint32_t packed[R];
+        if constexpr (NARROW) {
+            uint4 x[R];
 #pragma unroll
             for (int jj = 0; jj < R; ++jj)
-                if (sp[jj] != nullptr && g < groups) packed[jj] = *reinterpret_cast<const uint32_t *>(sp[jj] + g * 4);
+                x[jj] = sp[jj] != nullptr && lane * 16 < p.host_row_bytes ? *(reinterpret_cast<const uint4 *>(sp[jj]) + lane)
+                                                                          : make_uint4(0u, 0u, 0u, 0u);
+            // word g of a row is component g & 3 of lane g >> 2; the scale is word `groups`
+            auto word = [&](const uint4 &v, int g) {
+                const uint32_t a = __shfl_sync(kFull, v.x, g >> 2), b = __shfl_sync(kFull, v.y, g >> 2);
+                const uint32_t c = __shfl_sync(kFull, v.z, g >> 2), d = __shfl_sync(kFull, v.w, g >> 2);
+                return (g & 2) ? ((g & 1) ? d : c) : ((g & 1) ? b : a);
+            };
 #pragma unroll
             for (int jj = 0; jj < R; ++jj) {
-                if (sp[jj] != nullptr && g < groups) {
-                    float4 o;
-                    o.x = __fmul_rn(decode_code<CODEC>((uint8_t)(packed[jj])), scale[jj]);
-                    o.y = __fmul_rn(decode_code<CODEC>((uint8_t)(packed[jj] >> 8)), scale[jj]);
-                    o.z = __fmul_rn(decode_code<CODEC>((uint8_t)(packed[jj] >> 16)), scale[jj]);
-                    o.w = __fmul_rn(decode_code<CODEC>((uint8_t)(packed[jj] >> 24)), scale[jj]);
-                    __stcs(reinterpret_cast<float4 *>(dp[jj]) + g, o);
+                const float scale = __uint_as_float(word(x[jj], groups));
+                for (int g0 = 0; g0 < groups; g0 += 32) {
+                    const int g = g0 + lane;
+                    const uint32_t packed = word(x[jj], g < groups ? g : groups);
+                    if (sp[jj] != nullptr && g < groups) __stcs(reinterpret_cast<float4 *>(dp[jj]) + g, decode_word<CODEC>(packed, scale));
                 }
+            }
+        } else {
+            float scale[R];
+#pragma unroll
+            for (int jj = 0; jj < R; ++jj)
+                if (sp[jj] != nullptr) scale[jj] = *reinterpret_cast<const float *>(sp[jj] + f);
+            for (int g0 = 0; g0 < groups; g0 += 32) {
+                const int g = g0 + lane;
+                uint32_t packed[R];
+#pragma unroll
+                for (int jj = 0; jj < R; ++jj)
+                    if (sp[jj] != nullptr && g < groups) packed[jj] = *reinterpret_cast<const uint32_t *>(sp[jj] + g * 4);
+#pragma unroll
+                for (int jj = 0; jj < R; ++jj)
+                    if (sp[jj] != nullptr && g < groups) __stcs(reinterpret_cast<float4 *>(dp[jj]) + g, decode_word<CODEC>(packed[jj], scale[jj]));
             }
         }
     }
@@ -657,6 +738,7 @@ template <int R>
 __global__ void __launch_bounds__(1024) gather_miss_kernel(MissParams p)
 {
     __shared__ int s_last;
+    miss_zero_hist(p);
     const int n = p.miss_count[0];
     const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
@@ -725,8 +807,7 @@ struct LruParams {
     int64_t *cache_index;
     unsigned long long *stats;
     int32_t row_bytes;
-    int2 *miss_rows;
-    int32_t *miss_count;
+    MissSink miss;
 };
 
 __device__ __forceinline__ int64_t lru_set(int32_t id, int64_t sets)
@@ -792,7 +873,7 @@ __global__ void __launch_bounds__(256) gather_lru_kernel(LruParams p)
         }
         if (mine) p.cache_index[off + r] = slot;
         if (p.stats != nullptr) count_where(cta_counts, where, lane);
-        const MissTicket ticket = miss_begin(p.miss_count, where, src, lane);
+        const MissTicket ticket = miss_begin(p.miss, id, where, src, lane);
         const int rows_here = min(rpw, n - c * rpw);
         uint8_t *dst_base = p.dst + (int64_t)(off + c * rpw) * p.row_bytes;
         for (int j0 = 0; j0 < rows_here; j0 += R) {
@@ -823,7 +904,7 @@ __global__ void __launch_bounds__(256) gather_lru_kernel(LruParams p)
                 }
             }
         }
-        miss_finish(p.miss_rows, ticket, off + r, id, where, lane);
+        miss_finish(p.miss, ticket, off + r, id, where, lane);
     }
     __syncthreads();
     if (p.stats != nullptr && threadIdx.x < 3 && cta_counts[threadIdx.x] != 0)
@@ -979,6 +1060,32 @@ static int segment_grid(const LegionPool *p, int32_t op_id, int64_t *rows_out, i
     return (int)(g64 < 1 ? 1 : (g64 > cap ? cap : g64));
 }
 
+// List of the pipe's misses.  By stretches (miss_order_kernel in front of the fetch) where the fetch is long: behind an
+// LRU cache it is tens of thousands of rows over the whole table.
+static MissSink miss_sink(LegionPool *p, const LegionCache *c)
+{
+    const int pipe = p->pipe;
+    MissSink m;
+    m.rows = p->miss_rows[pipe];
+    m.count = p->miss_count[pipe];
+    const bool by_stretch = c != nullptr && c->host_table != nullptr && c->kind == 1;
+    m.n_rows = c != nullptr ? (int32_t)c->n_nodes : 1;
+    m.shift = 0;
+    while (((m.n_rows - 1) >> m.shift) >= kMissStretches) ++m.shift;
+    m.hist = by_stretch ? p->miss_hist[pipe] : nullptr;
+    m.rank = by_stretch ? p->miss_rank[pipe] : nullptr;
+    p->miss_ordered[pipe] = by_stretch ? 1 : 0;
+    return m;
+}
+
+template <int CODEC>
+static void launch_quant(int grid, cudaStream_t s, const GatherParams &gp)
+{
+    if (gp.feature_len <= 128) gather_quant_kernel<CODEC, 1, 8><<<grid, 256, 0, s>>>(gp);
+    else if (gp.feature_len <= 256) gather_quant_kernel<CODEC, 2, 8><<<grid, 256, 0, s>>>(gp);
+    else gather_quant_kernel<CODEC, 4, 4><<<grid, 256, 0, s>>>(gp);
+}
+
 // Lookup + gather of every row that is served from GPU memory; rows served by the host table
 // are listed for launch_gather_misses.
 int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op_id)
@@ -1005,8 +1112,7 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
         lp.cache_index = p->cache_index[pipe];
         lp.stats = c->stats;
         lp.row_bytes = row_bytes;
-        lp.miss_rows = p->miss_rows[pipe];
-        lp.miss_count = p->miss_count[pipe];
+        lp.miss = miss_sink(p, c);
         int vpl = (row_bytes / 16 + 31) / 32;
         LG_ARG(vpl >= 1 && vpl <= 4, "row size above 2048 bytes is not supported by the lru gather");
         switch (vpl) {
@@ -1036,8 +1142,7 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
     gp.row_bytes = row_bytes;
     gp.slot_bytes = c ? c->slot_bytes : row_bytes;
     gp.feature_len = row_bytes / 4;
-    gp.miss_rows = p->miss_rows[pipe];
-    gp.miss_count = p->miss_count[pipe];
+    gp.miss = miss_sink(p, c);
     gp.err = p->ctl[pipe] + CTL_ERROR;
     // staged seed rows are only meaningful for a launch that starts at the seeds, over uncompressed rows
     const bool staged = p->stage_rows != nullptr && (op_id == kOpGatherAll || op_id == 1) && c != nullptr &&
@@ -1074,8 +1179,10 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
 
     if (c != nullptr && c->codec != LEGION_CODEC_RAW) {
         LG_ARG(gp.feature_len % 4 == 0, "compressed rows need a feature length that is a multiple of 4");
-        if (c->codec == LEGION_CODEC_INT8) gather_quant_kernel<LEGION_CODEC_INT8><<<grid, 256, 0, s>>>(gp);
-        else gather_quant_kernel<LEGION_CODEC_E4M3><<<grid, 256, 0, s>>>(gp);
+        // (see gather_quant_kernel)
+        const int qgrid = segment_grid(p, op_id, nullptr, 8, op_id == kOpGatherAll ? 2 : 8);
+        if (c->codec == LEGION_CODEC_INT8) launch_quant<LEGION_CODEC_INT8>(qgrid, s, gp);
+        else launch_quant<LEGION_CODEC_E4M3>(qgrid, s, gp);
         LG_LAUNCH_CHECK();
         return LEGION_OK;
     }
@@ -1141,8 +1248,23 @@ int launch_gather_misses(cudaStream_t s, LegionPool *p, LegionCache *c)
     int threads = g_miss_threads > 0 ? g_miss_threads : (many ? kMissThreads : 128);
     const int rows = g_miss_rows > 0 ? g_miss_rows : (many ? 4 : 1);
     int grid = (int)(g64 < 1 ? 1 : (g64 > cap ? cap : g64));
-    if (c->host_codec == LEGION_CODEC_INT8) gather_miss_quant_kernel<LEGION_CODEC_INT8, 8><<<grid, threads, 0, s>>>(mp);
-    else if (c->host_codec == LEGION_CODEC_E4M3) gather_miss_quant_kernel<LEGION_CODEC_E4M3, 8><<<grid, threads, 0, s>>>(mp);
+    mp.hist = p->miss_ordered[pipe] ? p->miss_hist[pipe] : nullptr;
+    if (p->miss_ordered[pipe]) {
+        const MissSink m = miss_sink(p, c);
+        const int64_t og = (p->max_nodes + 1023) / 1024;
+        miss_order_kernel<<<(int)(og > p->sm_count ? p->sm_count : og), 1024, 0, s>>>(m.rows, m.rank, m.count, m.hist, m.shift, m.n_rows,
+                                                                                    p->miss_sorted[pipe]);
+        LG_LAUNCH_CHECK();
+        mp.miss_rows = p->miss_sorted[pipe];
+    }
+    const bool narrow = mp.host_row_bytes <= 512 && ((uintptr_t)mp.host & 15) == 0;
+    if (c->host_codec == LEGION_CODEC_INT8) {
+        if (narrow) gather_miss_quant_kernel<LEGION_CODEC_INT8, 4, true><<<grid, threads, 0, s>>>(mp);
+        else gather_miss_quant_kernel<LEGION_CODEC_INT8, 4, false><<<grid, threads, 0, s>>>(mp);
+    } else if (c->host_codec == LEGION_CODEC_E4M3) {
+        if (narrow) gather_miss_quant_kernel<LEGION_CODEC_E4M3, 4, true><<<grid, threads, 0, s>>>(mp);
+        else gather_miss_quant_kernel<LEGION_CODEC_E4M3, 4, false><<<grid, threads, 0, s>>>(mp);
+    }
     else if (rows == 1) gather_miss_kernel<1><<<grid, threads, 0, s>>>(mp);
     else if (rows == 2) gather_miss_kernel<2><<<grid, threads, 0, s>>>(mp);
     else if (rows == 8) gather_miss_kernel<8><<<grid, threads, 0, s>>>(mp);
@@ -1268,8 +1390,7 @@ extern "C" int legion_gather_rows_noalloc(void *stream, int32_t dev_id, const in
     gp.row_bytes = row_bytes;
     gp.slot_bytes = row_bytes;
     gp.feature_len = row_bytes / 4;
-    gp.miss_rows = reinterpret_cast<int2 *>(scratch + kNaMissRows);
-    gp.miss_count = miss_count;
+    gp.miss = MissSink{ reinterpret_cast<int2 *>(scratch + kNaMissRows), miss_count, nullptr, nullptr, 0, 1 };
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id);
     if (sms <= 0) sms = 148;
@@ -1289,7 +1410,8 @@ extern "C" int legion_gather_rows_noalloc(void *stream, int32_t dev_id, const in
     LG_LAUNCH_CHECK();
     if (host_table != nullptr) {
         MissParams mp;
-        mp.miss_rows = gp.miss_rows;
+        mp.miss_rows = gp.miss.rows;
+        mp.hist = nullptr;
         mp.miss_count = miss_count;
         mp.ticket = miss_count + 4;
         mp.host = (const uint8_t *)host_table;

@@ -79,3 +79,40 @@ def test_vector_gather_rows_per_warp(oracle_mod, row_bytes, count):
         want = table[ids] if with_host else np.where(np.isin(ids, order[: n // 2])[:, None], table[ids], 0)
         np.testing.assert_array_equal(out.cpu().numpy(), want)
     rig.close()
+
+
+@pytest.mark.parametrize("codec", [L.CODEC_INT8, L.CODEC_E4M3])
+@pytest.mark.parametrize("feat_len", [4, 100, 124, 128, 132, 256, 260, 508, 512, 772])
+@pytest.mark.parametrize("host_codec", [False, True])
+def test_compressed_gather_row_lengths(oracle_mod, codec, feat_len, host_codec):
+    """Row lengths around 128 and 256 codes (words per lane), 508 codes (rows that one 16-byte load per lane holds) and
+    lists of 1 to 33 rows and more; a third of the rows is cached.  Decoding is one multiplication: bits equal the host's."""
+    import torch
+    rng = np.random.default_rng(feat_len)
+    n = 900
+    table = rng.standard_normal((n, feat_len)).astype(np.float32)
+    stored = oracle_mod.quant_rows(table, codec)
+    plain = oracle_mod.dequant_rows(stored, feat_len, codec)
+    order = rng.permutation(n).astype(np.int32)
+    cached = np.isin(np.arange(n), order[: n // 3])
+    want = plain if host_codec else np.where(cached[:, None], plain, table)
+    for count in (1, 33, 700):
+        ids = rng.integers(0, n, count).astype(np.int32)
+        d_ids = torch.from_numpy(ids).cuda()
+        lab = torch.zeros(count, dtype=torch.int32, device="cuda")
+        host = torch.from_numpy(stored if host_codec else table).pin_memory()
+        f = L.FeatureStorage(0, n, feat_len * 4, host)
+        f.set_split(L.TRAINMODE, d_ids, lab)
+        cache = L.UnifiedCache(0, n, feat_len * 4, n // 3, codec=codec)
+        if host_codec:
+            cache.set_host_codec(codec)
+        cache.fill_static(torch.from_numpy(order).cuda(), host)
+        pool = L.MemoryPool(0, count, [], feat_len * 4, 1)
+        pool.set_batch(0, L.TRAINMODE, 0, 0)
+        L.BatchGenerate(None, f, cache, pool, count, 0, 0, 0, L.TRAINMODE, False, 0)
+        L.FeatureCacheLookup(None, cache, pool, 1, 0)
+        got = pool.read(L.BUF_FEATURES, 0, count * feat_len, np.float32).reshape(count, feat_len)
+        np.testing.assert_array_equal(got, want[ids])
+        st = cache.stats()
+        assert st["local_hits"] == cached[ids].sum() and st["misses"] == count - cached[ids].sum()
+        pool.close(); cache.close(); f.close()
