@@ -418,6 +418,34 @@ extern "C" int legion_cache_hotness_order(int32_t dev_id, const uint32_t *counts
     return rc;
 }
 
+// *missing = table entries that do not name a row of a partition of `capacity` rows.
+__global__ void count_missing_kernel(const int32_t *__restrict__ lut, int64_t n, int32_t capacity, int32_t *missing)
+{
+    int bad = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        if (lut[i] < 0 || lut[i] >= capacity) ++bad;
+    if (bad != 0) atomicAdd(missing, bad);
+}
+
+// Sets holds_all from the table just built.  Only a clique of one whose capacity covers the nodes is looked at.
+static int find_holds_all(LegionCache *c, int64_t n_cached, int sms, cudaStream_t s)
+{
+    if (c->kg != 1 || n_cached < c->n_nodes) return LEGION_OK;
+    int32_t *d = nullptr, missing = 1;
+    LG_CUDA(cudaMalloc(&d, sizeof(*d)));
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(*d), s);
+    if (e == cudaSuccess) {
+        count_missing_kernel<<<grid_stride(c->n_nodes, sms), 256, 0, s>>>(c->lut, c->n_nodes, c->capacity, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&missing, d, sizeof(missing), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaFree(d);
+    LG_CUDA(e);
+    c->holds_all = missing == 0 ? 1 : 0;
+    return LEGION_OK;
+}
+
 extern "C" int legion_cache_fill_static_rows(LegionCache *c, const int32_t *order_dev, int64_t n_order,
                                              const void *host_table, const int32_t *row_of_id_dev, void *stream)
 {
@@ -426,6 +454,7 @@ extern "C" int legion_cache_fill_static_rows(LegionCache *c, const int32_t *orde
     LG_CUDA(cudaSetDevice(c->dev_id));
     cudaStream_t s = (cudaStream_t)stream;
     c->host_table = host_table;
+    c->holds_all = 0;
     int sms = sm_count_of(c->dev_id);
     int64_t n_cached = (int64_t)c->capacity * c->kg;
     if (n_cached > n_order) n_cached = n_order;
@@ -458,7 +487,7 @@ extern "C" int legion_cache_fill_static_rows(LegionCache *c, const int32_t *orde
     }
     LG_CUDA(cudaStreamSynchronize(s));
     c->fill_gen += 1;
-    return LEGION_OK;
+    return find_holds_all(c, n_cached, sms, s);
 }
 
 extern "C" int legion_cache_add_replicas(LegionCache *c, const int32_t *order_dev, int64_t n_order, int64_t n_rows,

@@ -152,6 +152,7 @@ struct LegionCache {
     int32_t replica_rows;              // rows of part[kg] (legion_cache_add_replicas)
     int32_t fill_by_caller;            // set while legion_cache_place_static builds the table without copying rows
     int64_t fill_gen;                  // counts the changes of the lookup table (fill, replicas)
+    int32_t holds_all;                 // every node has a row in this GPU's own partition: no lookup can miss
     legion::VmmBlock own_block;        // set when part[ki] is shareable memory (clique of more than one GPU)
     legion::VmmBlock peer_block[LEGION_MAX_DEVICE];  // partitions mapped from other processes
     // lru
@@ -256,6 +257,7 @@ int launch_sample_hop(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32
 int launch_gather(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op_id);
 int launch_publish(cudaStream_t s, LegionPool *p);
 int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op_id);
+bool cache_may_miss(const LegionCache *c);
 int launch_gather_misses(cudaStream_t s, LegionPool *p, LegionCache *c);
 int launch_lru_insert(cudaStream_t s, LegionPool *p, LegionCache *c);
 int launch_hotness(cudaStream_t s, LegionPool *p, uint32_t *counts);

@@ -315,7 +315,7 @@ static int issue_back(LegionRunner *r)
 {
     LegionPool *p = r->pool;
     LegionCache *c = r->cache;
-    if (c != nullptr && c->host_table != nullptr) {
+    if (cache_may_miss(c)) {
         EvPair m = { nullptr, nullptr };
         if (r->time_kernels && r->miss_ev.size() < 8192) {
             m.a = take_event(r);
@@ -544,16 +544,24 @@ static int issue_rest(LegionRunner *r, int pipe, int32_t host_seeds, bool bound,
         LG_CUDA(cudaMemcpyAsync(hc, p->node_counter[pipe], 64, cudaMemcpyDeviceToHost, front));
         LG_CUDA(cudaMemcpyAsync(hc + 16, p->edge_counter[pipe], 64, cudaMemcpyDeviceToHost, front));
     }
-    LG_CUDA(cudaEventRecord(r->hit_done[pipe], front));
-    r->hit_recorded[pipe] = true;
-    LG_CUDA(cudaStreamWaitEvent(r->s_miss, r->hit_done[pipe], 0));
-    rc = issue_back(r);
-    if (rc != LEGION_OK) return rc;
+    // With rows to fetch or a cache to maintain the batch ends on s_miss, else with its gather: a hop to the other
+    // stream and back is 4-5 us of a small batch.
+    const bool back = lru || cache_may_miss(c);
+    cudaStream_t last = back ? r->s_miss : front;
+    if (back || r->seed_rows[pipe] != nullptr) {
+        LG_CUDA(cudaEventRecord(r->hit_done[pipe], front));
+        r->hit_recorded[pipe] = true;
+    }
+    if (back) {
+        LG_CUDA(cudaStreamWaitEvent(r->s_miss, r->hit_done[pipe], 0));
+        rc = issue_back(r);
+        if (rc != LEGION_OK) return rc;
+    }
     // (the export of a bound batch is waited for where it matters -- by collect, and by the batch that samples
     // ahead on this pipe -- not here: the fetch stream is shared by all batches and must not idle behind a copy)
-    LG_CUDA(cudaEventRecord(r->pipe_done[pipe], r->s_miss));
+    LG_CUDA(cudaEventRecord(r->pipe_done[pipe], last));
     if (p->slots < p->pipes) {
-        LG_CUDA(cudaEventRecord(r->slot_done[slot], r->s_miss));
+        LG_CUDA(cudaEventRecord(r->slot_done[slot], last));
         r->slot_busy[slot] = true;
     }
     if (lru) c->clock += 1;
@@ -943,7 +951,12 @@ extern "C" int legion_runner_sync(LegionRunner *r)
         int frc = flush_deferred(r);
         if (frc != LEGION_OK) return frc;
     }
-    if (r->open_window) LG_CUDA(cudaEventRecord(r->t_end, r->s_miss));  // the miss stream ends every batch
+    if (r->open_window) {
+        // behind the end of every batch, on whichever stream it is
+        for (int i = 0; i < LEGION_MAX_PIPES; ++i)
+            if (r->pipe_busy[i]) LG_CUDA(cudaStreamWaitEvent(r->s_miss, r->pipe_done[i], 0));
+        LG_CUDA(cudaEventRecord(r->t_end, r->s_miss));
+    }
     LG_CUDA(cudaStreamSynchronize(r->s_sample));
     LG_CUDA(cudaStreamSynchronize(r->s_gather));
     LG_CUDA(cudaStreamSynchronize(r->s_miss));

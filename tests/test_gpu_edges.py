@@ -116,3 +116,26 @@ def test_compressed_gather_row_lengths(oracle_mod, codec, feat_len, host_codec):
         st = cache.stats()
         assert st["local_hits"] == cached[ids].sum() and st["misses"] == count - cached[ids].sum()
         pool.close(); cache.close(); f.close()
+
+
+def test_cache_that_holds_every_node_needs_no_fetch(oracle_mod):
+    """A cache with room for every node skips the fetch of misses; one whose order names a node twice, and so leaves another
+    out, must not, nor one that is filled again with fewer nodes."""
+    import torch
+    rng = np.random.default_rng(5)
+    n, row_bytes, count = 700, 64, 900
+    table = rng.integers(0, 256, (n, row_bytes)).astype(np.uint8)
+    ids = rng.integers(0, n, count).astype(np.int32)
+    order = rng.permutation(n).astype(np.int32)
+    twice = order.copy()
+    twice[-1] = twice[0]
+    for o, held in ((order, n), (twice, n - 1), (order[: n // 2], n // 2), (order, n)):
+        rig = Rig(table, ids, count, capacity=n, order=o)
+        for _ in range(2):
+            np.testing.assert_array_equal(rig.gather(0)[1], table[ids])
+        st = rig.cache.stats()
+        miss = (~np.isin(ids, o)).sum()
+        assert st["misses"] == 2 * miss and st["local_hits"] == 2 * (count - miss) and (miss == 0) == (held == n)
+        rig.cache.fill_static(torch.from_numpy(order[:10].copy()).cuda(), rig.h_table)
+        np.testing.assert_array_equal(rig.gather(0)[1], table[ids])
+        rig.close()
