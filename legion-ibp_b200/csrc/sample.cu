@@ -544,8 +544,14 @@ int g_pdl = pdl_from_env();
 // (legion_set_tunable "map_front_shift")
 int g_map_front_shift = -1;
 
+// Without the tunable, batches that have the GPU to themselves are launched this way too: pools of one pipe, and small
+// ones, whose launches are mostly start and drain.  Measured: 1,237 seeds,
+// [15,10], through the operators 115 -> 107 us, 32 seeds, [10,5], 80.5 -> 79.7; with four pipes of 800 seeds, [25,10], whose
+// kernels fill each other's gaps, nothing.
+constexpr int64_t kDependentNodes = 1 << 16;
+
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_dep(void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args... args)
+static cudaError_t launch_dep(const LegionPool *p, void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -555,8 +561,9 @@ static cudaError_t launch_dep(void (*kernel)(KArgs...), int grid, int block, cud
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = g_pdl ? at : nullptr;
-    cfg.numAttrs = g_pdl ? 1 : 0;
+    const bool dependent = g_pdl || p->pipes == 1 || p->max_nodes <= kDependentNodes;
+    cfg.attrs = dependent ? at : nullptr;
+    cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
@@ -612,7 +619,7 @@ static cudaError_t launch_hop_sample(cudaStream_t s, LegionPool *p, const Legion
                                      int64_t inputs, int tile_shift)
 {
     const int pipe = p->pipe;
-    return launch_dep(hop_sample_kernel<G>, grid_for(inputs, 8 * (32 / G), p->sm_count * 6), 256, s, g->indptr, g->indices, p->ids[pipe], fanout,
+    return launch_dep(p, hop_sample_kernel<G>, grid_for(inputs, 8 * (32 / G), p->sm_count * 6), 256, s, g->indptr, g->indices, p->ids[pipe], fanout,
                       (uint32_t)hop, p->bctl[pipe], p->edge_rec[pipe], p->map[pipe], MapDims{ p->map_front_mask, p->map_mask },
                       p->ctl[pipe], p->node_counter[pipe], p->edge_cnt[pipe], p->tile_state[pipe], tile_shift,
                       p->max_hop_edges);
@@ -622,7 +629,7 @@ template <int IPT>
 static cudaError_t launch_hop_finish(cudaStream_t s, LegionPool *p, int32_t fanout, int32_t hop, int32_t op_id, int64_t edges)
 {
     const int pipe = p->pipe;
-    return launch_dep(hop_finish_kernel<IPT>, grid_for(edges, kScanThreads * IPT, p->sm_count * 8), kScanThreads, s, p->edge_rec[pipe],
+    return launch_dep(p, hop_finish_kernel<IPT>, grid_for(edges, kScanThreads * IPT, p->sm_count * 8), kScanThreads, s, p->edge_rec[pipe],
                       fanout, p->tile_state[pipe], p->ids[pipe], p->map[pipe], p->src_global[pipe], p->agg_src[pipe],
                       p->agg_dst[pipe], p->ctl[pipe], p->node_counter[pipe], p->edge_counter[pipe], op_id, p->bctl[pipe],
                       hop + 1 == p->hop_num ? 1 : 0, p->max_nodes, p->max_edges);
