@@ -125,7 +125,7 @@ def test_cache_that_holds_every_node_needs_no_fetch(oracle_mod):
     rng = np.random.default_rng(5)
     n, row_bytes, count = 700, 64, 900
     table = rng.integers(0, 256, (n, row_bytes)).astype(np.uint8)
-    ids = rng.integers(0, n, count).astype(np.int32)
+    ids = np.concatenate([rng.permutation(n), rng.integers(0, n, count - n)]).astype(np.int32)   # every node is asked for
     order = rng.permutation(n).astype(np.int32)
     twice = order.copy()
     twice[-1] = twice[0]
