@@ -255,7 +255,6 @@ const void *batch_start_kernel_address();
 int launch_sample_hop(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop,
                       int32_t op_id);
 int launch_gather(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op_id);
-int launch_publish(cudaStream_t s, LegionPool *p);
 int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op_id);
 bool cache_may_miss(const LegionCache *c);
 int launch_gather_misses(cudaStream_t s, LegionPool *p, LegionCache *c);

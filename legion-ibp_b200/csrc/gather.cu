@@ -30,9 +30,40 @@ struct MissSink {
     int32_t shift, n_rows;  // rows of the table
 };
 
+// Hand-off of a batch that was sampled ahead.  A pool with fewer hand-off slots than pipes samples into private
+// buffers; when the batch's turn comes, its block structure (ids, labels, both edge lists, both counter arrays: ~3 MB for a
+// paper100M-shaped batch) is copied into the slot that the consumer reads (the buffers of engine/ipc_service.cu:163-169).
+// Sizes are read from the counters on the device.  All of the grid takes part.
+struct Publish {
+    const int32_t *ids, *labels, *src, *dst, *nc, *ec;
+    int32_t *o_ids, *o_labels, *o_src, *o_dst, *o_nc, *o_ec;  // o_ids nullptr: nothing to hand off
+};
+__device__ __forceinline__ void publish_copy(const Publish &p)
+{
+    const int hops = p.nc[LEGION_INTRABATCH_CON * 3 - 1];
+    const int n = p.nc[LEGION_INTRABATCH_CON * 3 + hops];
+    const int n_lab = p.nc[LEGION_INTRABATCH_CON * 3];
+    const int e = p.ec[0] + p.ec[1];
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    // every array is padded to whole 1024-element tiles, so whole 16-byte vectors may be copied
+    for (int i = tid; i * 4 < n; i += step) reinterpret_cast<int4 *>(p.o_ids)[i] = reinterpret_cast<const int4 *>(p.ids)[i];
+    for (int i = tid; i * 4 < e; i += step) {
+        const int4 a = reinterpret_cast<const int4 *>(p.src)[i], b = reinterpret_cast<const int4 *>(p.dst)[i];
+        reinterpret_cast<int4 *>(p.o_src)[i] = a;
+        reinterpret_cast<int4 *>(p.o_dst)[i] = b;
+    }
+    for (int i = tid; i < n_lab; i += step) p.o_labels[i] = p.labels[i];
+    if (blockIdx.x == 0 && threadIdx.x < 16) {
+        // words 2 and 3 are the snapshot of the lookup, which segment_of leaves there
+        if (threadIdx.x != 2 && threadIdx.x != 3) p.o_nc[threadIdx.x] = p.nc[threadIdx.x];
+        p.o_ec[threadIdx.x] = p.ec[threadIdx.x];
+    }
+}
+
 struct GatherParams {
     const int32_t *ids;
     int32_t *nc;  // node_counter of the pipe
+    int32_t *nc_out;  // where the snapshot of the lookup goes: the same, or the hand-off slot's
     int32_t op_id;
     const int32_t *lut;
     int32_t capacity, kg, ki;
@@ -54,6 +85,7 @@ struct GatherParams {
     int32_t n_rows;      // rows of a list of the caller's own; -1: the segment of op_id in the counters
     int32_t rows_per_warp; // fixed by a tunable; 0: chosen by the length of the list
     MissSink miss;
+    Publish pub;
 };
 
 // A missed row that sits in the batch's staging area is served from there like a cached row; `where` 4 keeps
@@ -78,7 +110,7 @@ __device__ __forceinline__ const uint8_t *shfl_ptr(const uint8_t *p, int src)
 // the cumulative counts nc[9+h], which are written once per batch, so that a gather may overlap
 // the sampling of the next hop on another stream.  Block 0 also leaves the (offset, size)
 // snapshot that counter_update writes for a lookup op (operator_impl.cu:85-87).
-__device__ __forceinline__ void segment_of(int32_t *nc, int op_id, int &off, int &n, int n_rows = -1)
+__device__ __forceinline__ void segment_of(const int32_t *nc, int32_t *nc_out, int op_id, int &off, int &n, int n_rows = -1)
 {
     if (n_rows >= 0) {
         off = 0;
@@ -93,8 +125,8 @@ __device__ __forceinline__ void segment_of(int32_t *nc, int op_id, int &off, int
         n = nc[LEGION_INTRABATCH_CON * 3 + hops];
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             const int last = hops > 0 ? nc[LEGION_INTRABATCH_CON * 3 + hops - 1] : 0;
-            nc[2] = last;
-            nc[3] = n - last;
+            nc_out[2] = last;
+            nc_out[3] = n - last;
         }
         return;
     }
@@ -102,8 +134,8 @@ __device__ __forceinline__ void segment_of(int32_t *nc, int op_id, int &off, int
     off = h > 0 ? nc[LEGION_INTRABATCH_CON * 3 + h - 1] : 0;
     n = nc[LEGION_INTRABATCH_CON * 3 + h] - off;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        nc[(op_id % LEGION_INTRABATCH_CON) * 2] = off;
-        nc[(op_id % LEGION_INTRABATCH_CON) * 2 + 1] = n;
+        nc_out[(op_id % LEGION_INTRABATCH_CON) * 2] = off;
+        nc_out[(op_id % LEGION_INTRABATCH_CON) * 2 + 1] = n;
     }
 }
 
@@ -269,8 +301,9 @@ __global__ void __launch_bounds__(256) gather_vec_kernel(GatherParams p)
     __shared__ int cta_counts[3];
     if (threadIdx.x < 3) cta_counts[threadIdx.x] = 0;
     __syncthreads();
+    if (p.pub.o_ids != nullptr) publish_copy(p.pub);
     int off, n;
-    segment_of(p.nc, p.op_id, off, n, p.n_rows);
+    segment_of(p.nc, p.nc_out, p.op_id, off, n, p.n_rows);
     const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     const int row_vec = p.row_bytes >> 4;
@@ -365,7 +398,7 @@ __global__ void __launch_bounds__(kBulkWarps * 32) gather_bulk_kernel(GatherPara
     extern __shared__ __align__(128) uint8_t bulk_smem[];          // [warp][32 rows][row_bytes]
     __shared__ __align__(8) unsigned long long bars[kBulkWarps];
     int off, n;
-    segment_of(p.nc, p.op_id, off, n);
+    segment_of(p.nc, p.nc_out, p.op_id, off, n);
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
@@ -447,8 +480,9 @@ __global__ void __launch_bounds__(256) gather_flat_kernel(GatherParams p)
     __shared__ int cta_counts[3];
     if (threadIdx.x < 3) cta_counts[threadIdx.x] = 0;
     __syncthreads();
+    if (p.pub.o_ids != nullptr) publish_copy(p.pub);
     int off, n;
-    segment_of(p.nc, p.op_id, off, n, p.n_rows);
+    segment_of(p.nc, p.nc_out, p.op_id, off, n, p.n_rows);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     const int rpw = rows_per_warp_for(n, n_warps, 4);
@@ -530,8 +564,9 @@ __global__ void __launch_bounds__(256) gather_quant_kernel(GatherParams p)
     __shared__ int cta_counts[3];
     if (threadIdx.x < 3) cta_counts[threadIdx.x] = 0;
     __syncthreads();
+    if (p.pub.o_ids != nullptr) publish_copy(p.pub);
     int off, n;
-    segment_of(p.nc, p.op_id, off, n);
+    segment_of(p.nc, p.nc_out, p.op_id, off, n);
     const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     const int f = p.feature_len, groups = f >> 2;
@@ -845,7 +880,7 @@ __global__ void __launch_bounds__(256) gather_lru_kernel(LruParams p)
     if (threadIdx.x < 3) cta_counts[threadIdx.x] = 0;
     __syncthreads();
     int off, n;
-    segment_of(p.nc, p.op_id, off, n);
+    segment_of(p.nc, p.nc, p.op_id, off, n);
     const int lane = threadIdx.x & 31;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     const int row_vec = p.row_bytes >> 4;
@@ -1011,6 +1046,8 @@ lru_commit_kernel(const int32_t *__restrict__ ids, const int32_t *__restrict__ n
 
 // ---- launchers ------------------------------------------------------------------------------------------
 
+__global__ void __launch_bounds__(256) publish_kernel(Publish p) { publish_copy(p); }
+
 template <int VPL, int R>
 static void launch_vec(int grid, cudaStream_t s, const GatherParams &gp)
 {
@@ -1127,7 +1164,7 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
 
     GatherParams gp;
     gp.ids = p->ids[pipe];
-    gp.nc = p->pub_nc[pipe % p->slots];  // the hand-off slot's counters (the pipe's own unless it samples ahead)
+    gp.nc = gp.nc_out = p->pub_nc[pipe % p->slots];  // the hand-off slot's counters (the pipe's own unless it samples ahead)
     gp.op_id = op_id;
     gp.lut = c ? c->lut : nullptr;
     gp.capacity = c ? (c->capacity > 0 ? c->capacity : 1) : 1;
@@ -1153,6 +1190,21 @@ int launch_gather_hits(cudaStream_t s, LegionPool *p, LegionCache *c, int32_t op
     gp.stage_n = staged ? p->stage_n : 0;
     gp.n_rows = -1;
     gp.rows_per_warp = 0;
+
+    // The gather over a batch that was sampled ahead also hands its block structure over; a launch of its own for that
+    // was 4 us of every batch.  The bulk-copy engine keeps the two apart.
+    gp.pub.o_ids = nullptr;
+    if (p->slots < p->pipes && op_id == kOpGatherAll) {
+        const int slot = pipe % p->slots;
+        gp.pub = Publish{ p->ids[pipe], p->labels[pipe], p->agg_src[pipe], p->agg_dst[pipe], p->node_counter[pipe], p->edge_counter[pipe],
+                          p->pub_ids[slot], p->pub_labels[slot], p->pub_agg_src[slot], p->pub_agg_dst[slot], p->pub_nc[slot], p->pub_ec[slot] };
+        if (g_gather_engine == 1) {
+            publish_kernel<<<p->sm_count * 2, 256, 0, s>>>(gp.pub);
+            LG_LAUNCH_CHECK();
+            gp.pub.o_ids = nullptr;
+        }
+        gp.nc = p->node_counter[pipe];
+    }
 
     // the bulk-copy engine has only ever read this GPU's own memory: a clique of more than one GPU keeps the register path
     if (g_gather_engine == 1 && gp.kg == 1 && (c == nullptr || c->codec == LEGION_CODEC_RAW) && row_bytes % 16 == 0 &&
@@ -1374,7 +1426,8 @@ extern "C" int legion_gather_rows_noalloc(void *stream, int32_t dev_id, const in
 
     GatherParams gp;
     gp.ids = ids_dev;
-    gp.nc = nullptr;
+    gp.nc = gp.nc_out = nullptr;
+    gp.pub.o_ids = nullptr;
     gp.op_id = 1;
     gp.n_rows = (int32_t)n_rows;
     gp.rows_per_warp = 0;

@@ -520,10 +520,8 @@ static int issue_rest(LegionRunner *r, int pipe, int32_t host_seeds, bool bound,
     const int slot = pipe % p->slots;
     if (p->slots < p->pipes) {
         // the batch was sampled ahead into the pipe's private buffers: once the batch that used the hand-off slot
-        // before has left it, the block structure is copied into the slot, and the gather fills the slot's rows
+        // before has left it, the gather fills the slot's rows and copies the block structure into the slot
         if (r->slot_busy[slot] && !pipe_was_synced) LG_CUDA(cudaStreamWaitEvent(front, r->slot_done[slot], 0));
-        rc = launch_publish(front, p);
-        if (rc != LEGION_OK) return rc;
     }
     if (r->pipe_stage[pipe] != nullptr) {
         const SeedStage *st = r->pipe_stage[pipe];

@@ -654,44 +654,4 @@ int launch_sample_hop(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32
     return LEGION_OK;
 }
 
-// ---- hand-off of a batch that was sampled ahead ------------------------------------------------------------------
-// A pool with fewer hand-off slots than pipes samples into private buffers; when the batch's turn comes, its
-// block structure (ids, labels, both edge lists, both counter arrays: ~3 MB for a paper100M-shaped batch) is
-// copied into the slot that the consumer reads (the buffers of engine/ipc_service.cu:163-169).  Sizes are read
-// from the counters on the device.
-__global__ void __launch_bounds__(256)
-publish_kernel(const int32_t *__restrict__ ids, const int32_t *__restrict__ labels, const int32_t *__restrict__ src,
-               const int32_t *__restrict__ dst, const int32_t *__restrict__ nc, const int32_t *__restrict__ ec,
-               int32_t *o_ids, int32_t *o_labels, int32_t *o_src, int32_t *o_dst, int32_t *o_nc, int32_t *o_ec)
-{
-    const int hops = nc[LEGION_INTRABATCH_CON * 3 - 1];
-    const int n = nc[LEGION_INTRABATCH_CON * 3 + hops];
-    const int n_lab = nc[LEGION_INTRABATCH_CON * 3];
-    const int e = ec[0] + ec[1];
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-    // every array is padded to whole 1024-element tiles, so whole 16-byte vectors may be copied
-    for (int i = tid; i * 4 < n; i += step) reinterpret_cast<int4 *>(o_ids)[i] = reinterpret_cast<const int4 *>(ids)[i];
-    for (int i = tid; i * 4 < e; i += step) {
-        reinterpret_cast<int4 *>(o_src)[i] = reinterpret_cast<const int4 *>(src)[i];
-        reinterpret_cast<int4 *>(o_dst)[i] = reinterpret_cast<const int4 *>(dst)[i];
-    }
-    for (int i = tid; i < n_lab; i += step) o_labels[i] = labels[i];
-    if (blockIdx.x == 0 && threadIdx.x < 16) {
-        o_nc[threadIdx.x] = nc[threadIdx.x];
-        o_ec[threadIdx.x] = ec[threadIdx.x];
-    }
-}
-
-int launch_publish(cudaStream_t s, LegionPool *p)
-{
-    if (p->slots == p->pipes) return LEGION_OK;  // the pipe's buffers are the hand-off buffers
-    const int pipe = p->pipe, slot = pipe % p->slots;
-    publish_kernel<<<p->sm_count * 2, 256, 0, s>>>(p->ids[pipe], p->labels[pipe], p->agg_src[pipe], p->agg_dst[pipe],
-                                                   p->node_counter[pipe], p->edge_counter[pipe], p->pub_ids[slot],
-                                                   p->pub_labels[slot], p->pub_agg_src[slot], p->pub_agg_dst[slot],
-                                                   p->pub_nc[slot], p->pub_ec[slot]);
-    LG_LAUNCH_CHECK();
-    return LEGION_OK;
-}
-
 }  // namespace legion
