@@ -1101,7 +1101,10 @@ def main():
 
     if rank == 0:
         hops = len(cfg["fanout"])
-        per_batch = 1 + 4 * hops + 1 + (1 if not striped else 0) + (3 if lru_ways else 0)
+        # start, two per hop, gather; the fetch of missed rows where there can be any; an LRU cache orders its list and
+        # inserts with two more
+        fetch = not striped and (world > 1 or lru_ways or cfg["cache_frac"] < 1.0)
+        per_batch = 1 + 2 * hops + 1 + (1 if fetch else 0) + (3 if lru_ways else 0)
         line = {"metric": "sampled+gathered mini-batches/sec", "value": value, "unit": "batches/s",
                 "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
                 "ms_per_step": ms_total / args.steps, "higher_is_better": True, "scaling": "weak",

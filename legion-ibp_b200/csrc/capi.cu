@@ -224,7 +224,7 @@ extern "C" int legion_pool_create_ahead(LegionPool **out, int32_t dev_id, int32_
         if (e == cudaSuccess) e = dmalloc(&p->src_global[i], pad_edges);
         if (e == cudaSuccess) e = dmalloc(&p->map[i], (int64_t)front + cap);
         if (e == cudaSuccess) e = dmalloc(&p->edge_rec[i], pad_hop_edges);
-        if (e == cudaSuccess) e = dmalloc(&p->tile_state[i], pad_hop_edges / kScanThreads);
+        if (e == cudaSuccess) e = dmalloc(&p->tile_state[i], pad_hop_edges / kTile);
         if (e == cudaSuccess) e = dmalloc(&p->edge_cnt[i], (hop_num > 0 ? hop_num : 1) * pad_nodes);
         if (e == cudaSuccess) e = dmalloc(&p->lru_victim[i], pad_nodes);
         if (e == cudaSuccess) e = dmalloc(&p->ctl[i], CTL_WORDS);

@@ -35,7 +35,7 @@ void set_error(const char *fmt, ...);
 #define LG_LAUNCH_CHECK() LG_CUDA(cudaGetLastError())
 
 // ---- device-side batch state --------------------------------------------------------------
-// Tile = number of entries one CTA scans at a time (256 in small hops).
+// Tile = number of entries one CTA scans at a time.
 constexpr int kTile = 1024;
 constexpr int kScanThreads = 256;
 

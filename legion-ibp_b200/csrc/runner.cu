@@ -10,7 +10,7 @@
 // launch per batch behind the last gather so that the link sees one long burst instead of three
 // short ones.  The gather of hop h overlaps the sampling of hop h+1.
 //
-// A batch is ~15 small launches, so issuing it from the host costs more than running it.  Every
+// A batch is 6 to 10 small launches, so issuing it from the host costs more than running it.  Every
 // size lives on the device and the per-batch parameters are written by the first kernel, so the
 // sampling sequence of one pipe is captured once into a CUDA graph; a batch is then one parameter
 // update of that first node, one graph launch, the gather launch and the host-link fetch.  The two

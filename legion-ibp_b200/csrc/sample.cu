@@ -265,8 +265,7 @@ template <int G>
 __global__ void __launch_bounds__(256, 6)
 hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict__ indices, const int32_t *ids,
                   int32_t fanout, uint32_t hop, const BatchCtl *__restrict__ b, int2 *rec, MapSlot *map, MapDims mask,
-                  int32_t *ctl, const int32_t *nc, uint8_t *edge_cnt, uint32_t *tile_state, int tile_shift,
-                  int64_t max_entries)
+                  int32_t *ctl, const int32_t *nc, uint8_t *edge_cnt, uint32_t *tile_state, int64_t max_entries)
 {
     pdl_wait();
     pdl_trigger();
@@ -284,7 +283,7 @@ hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict_
     }
     const uint32_t k = (uint32_t)fanout;
     // the tiles that hop_finish_kernel is about to scan have not been counted yet
-    for (int t = tid, n_tiles = (n * fanout + (1 << tile_shift) - 1) >> tile_shift; t < n_tiles; t += n_threads) tile_state[t] = 0;
+    for (int t = tid, n_tiles = (n * fanout + kTile - 1) / kTile; t < n_tiles; t += n_threads) tile_state[t] = 0;
     const uint32_t batch_id = b->global_batch, k0 = b->k0, k1 = b->k1;
     const int max_rounds = b->max_rounds;
     const int n_limit = b->n_nodes;
@@ -400,7 +399,7 @@ __device__ __forceinline__ void advance_counters(int word, int c, int e, int n0,
     }
 }
 
-// One pass over the entries of a hop, in tiles of 256 * IPT.  A CTA counts its tile's edges and the entries that
+// One pass over the entries of a hop, in tiles of 1024.  A CTA counts its tile's edges and the entries that
 // reached a node first, publishes both counts, adds up the counts of the tiles before it (each CTA reads them all,
 // one word per tile, so nothing is passed from tile to tile) and places its edges and new nodes.
 // Tiles are handed out in order by a ticket and a CTA publishes its counts before it waits for others, so the
@@ -411,9 +410,9 @@ __device__ __forceinline__ void advance_counters(int word, int c, int e, int n0,
 // of the whole CTA, were 4 of the 9-11 us that the launch took on two tiles).
 // The local id of a node that another entry reached first is written to its map slot by that entry's CTA, which has
 // an earlier tile, or the same one.
-// Bound by L2 latency: record, map slot, counts, map slot.  IPT 1 where the hop is small (a tile for every SM),
-// 4 where it is large (four map reads of a thread in flight, fewer counts to add up).
-template <int IPT>
+// Bound by L2 latency: record, map slot, counts, map slot.  Four entries per thread: four map reads in flight and fewer
+// counts to add up.  (Tiles of 256 in small hops, for more CTAs: eight batches of 800 seeds, [25,10], 267 against 264 us,
+// and 295 where hop 2 used them too; one batch alone the same.)
 __global__ void __launch_bounds__(kScanThreads, 6)
 hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_state, int32_t *ids, MapSlot *map,
                   int32_t *src_global, int32_t *agg_src, int32_t *agg_dst, int32_t *ctl, int32_t *nc, int32_t *ec, int op_id,
@@ -421,7 +420,8 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
 {
     pdl_wait();
     pdl_trigger();
-    constexpr int TILE = kScanThreads * IPT;
+    constexpr int IPT = kTile / kScanThreads, TILE = kTile;
+    static_assert(IPT == 4, "records are read as two 16-byte vectors per thread");
     __shared__ int smem[kScanThreads / 32];
     __shared__ int s_edges[kScanThreads / 32], s_new[kScanThreads / 32];
     __shared__ int s_tile;
@@ -444,16 +444,11 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
         if (tile >= n_tiles) break;
         const int base = tile * TILE + threadIdx.x * IPT;
         int u[IPT], slot[IPT], val[IPT];
-        if constexpr (IPT == 4) {
-            // rec is padded to whole tiles
-            const int4 *r4 = reinterpret_cast<const int4 *>(rec + base);
-            const int4 r0 = __ldcs(r4), r1 = __ldcs(r4 + 1);
-            u[0] = r0.x; slot[0] = r0.y; u[1] = r0.z; slot[1] = r0.w;
-            u[2] = r1.x; slot[2] = r1.y; u[3] = r1.z; slot[3] = r1.w;
-        } else {
-            const int2 r = __ldcs(rec + base);
-            u[0] = r.x; slot[0] = r.y;
-        }
+        // rec is padded to whole tiles
+        const int4 *r4 = reinterpret_cast<const int4 *>(rec + base);
+        const int4 r0 = __ldcs(r4), r1 = __ldcs(r4 + 1);
+        u[0] = r0.x; slot[0] = r0.y; u[1] = r0.z; slot[1] = r0.w;
+        u[2] = r1.x; slot[2] = r1.y; u[3] = r1.z; slot[3] = r1.w;
 #pragma unroll
         for (int j = 0; j < IPT; ++j) {
             if (base + j >= total) slot[j] = -1;
@@ -616,20 +611,18 @@ int launch_batch_generate(cudaStream_t s, LegionPool *p, const BatchCtl &v)
 
 template <int G>
 static cudaError_t launch_hop_sample(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop,
-                                     int64_t inputs, int tile_shift)
+                                     int64_t inputs)
 {
     const int pipe = p->pipe;
     return launch_dep(p, hop_sample_kernel<G>, grid_for(inputs, 8 * (32 / G), p->sm_count * 6), 256, s, g->indptr, g->indices, p->ids[pipe], fanout,
                       (uint32_t)hop, p->bctl[pipe], p->edge_rec[pipe], p->map[pipe], MapDims{ p->map_front_mask, p->map_mask },
-                      p->ctl[pipe], p->node_counter[pipe], p->edge_cnt[pipe], p->tile_state[pipe], tile_shift,
-                      p->max_hop_edges);
+                      p->ctl[pipe], p->node_counter[pipe], p->edge_cnt[pipe], p->tile_state[pipe], p->max_hop_edges);
 }
 
-template <int IPT>
 static cudaError_t launch_hop_finish(cudaStream_t s, LegionPool *p, int32_t fanout, int32_t hop, int32_t op_id, int64_t edges)
 {
     const int pipe = p->pipe;
-    return launch_dep(p, hop_finish_kernel<IPT>, grid_for(edges, kScanThreads * IPT, p->sm_count * 8), kScanThreads, s, p->edge_rec[pipe],
+    return launch_dep(p, hop_finish_kernel, grid_for(edges, kTile, p->sm_count * 8), kScanThreads, s, p->edge_rec[pipe],
                       fanout, p->tile_state[pipe], p->ids[pipe], p->map[pipe], p->src_global[pipe], p->agg_src[pipe],
                       p->agg_dst[pipe], p->ctl[pipe], p->node_counter[pipe], p->edge_counter[pipe], op_id, p->bctl[pipe],
                       hop + 1 == p->hop_num ? 1 : 0, p->max_nodes, p->max_edges);
@@ -641,16 +634,12 @@ int launch_sample_hop(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32
     int64_t inputs = p->batch_size;
     for (int h = 0; h < hop; ++h) inputs += inputs * p->fanout[h];
     const int64_t edges = inputs * fanout;
-    const bool wide = edges > (int64_t)p->sm_count * kTile;  // more entries than one 1024-entry tile per SM
-    const int tile_shift = wide ? 10 : 8;
-    static_assert(kScanThreads == 256 && kTile == 1024, "tile shifts above assume 256-thread scans over 1024-item tiles");
     switch (group_lanes(fanout)) {
-    case 8: LG_CUDA(launch_hop_sample<8>(s, p, g, fanout, hop, inputs, tile_shift)); break;
-    case 16: LG_CUDA(launch_hop_sample<16>(s, p, g, fanout, hop, inputs, tile_shift)); break;
-    default: LG_CUDA(launch_hop_sample<32>(s, p, g, fanout, hop, inputs, tile_shift)); break;
+    case 8: LG_CUDA(launch_hop_sample<8>(s, p, g, fanout, hop, inputs)); break;
+    case 16: LG_CUDA(launch_hop_sample<16>(s, p, g, fanout, hop, inputs)); break;
+    default: LG_CUDA(launch_hop_sample<32>(s, p, g, fanout, hop, inputs)); break;
     }
-    if (wide) LG_CUDA(launch_hop_finish<4>(s, p, fanout, hop, op_id, edges));
-    else LG_CUDA(launch_hop_finish<1>(s, p, fanout, hop, op_id, edges));
+    LG_CUDA(launch_hop_finish(s, p, fanout, hop, op_id, edges));
     return LEGION_OK;
 }
 

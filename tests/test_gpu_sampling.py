@@ -260,7 +260,7 @@ def test_isolated_nodes_hubs_and_empty_topology(oracle_mod):
 @pytest.mark.parametrize("max_rounds", [1, 64])
 def test_lane_groups_and_scan_tiles(oracle_mod, fanout, batch, max_rounds):
     """Fanouts at the edges of the lane groups that share an input (8, 16, 32), degrees on both sides of the fanout and
-    of twice the fanout, batches around the scan's tiles of 256 entries; with one round nearly every draw goes
+    of twice the fanout, batches around the scan's tiles of 1024 entries; with one round nearly every draw goes
     through the lane-ordered fallback."""
     indptr, indices = small_graph(2500, 30000, 31)
     rng = np.random.default_rng(batch)
@@ -276,7 +276,7 @@ def test_lane_groups_and_scan_tiles(oracle_mod, fanout, batch, max_rounds):
 
 
 def test_large_hop_matches_host_replay(oracle_mod):
-    """A hop of more entries than one 1024-entry tile per SM, and more tiles than CTAs that run at once."""
+    """A hop of more 1024-entry tiles than CTAs that run at once."""
     indptr, indices = small_graph(150000, 4000000, 41)
     rng = np.random.default_rng(3)
     train = rng.permutation(150000)[:9000].astype(np.int32)
