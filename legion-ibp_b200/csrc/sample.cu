@@ -169,32 +169,6 @@ __device__ __forceinline__ int block_excl_scan(int x, int *total, int *smem)
     return wo + incl - x;
 }
 
-// literal restatement of counter_update (operator_impl.cu:58-91), executed by one thread
-__device__ __forceinline__ void counter_update(int32_t *nc, int32_t *ec, int op_id, int size, int hop_num)
-{
-    const int C = LEGION_INTRABATCH_CON;
-    if (op_id == 0) {
-        nc[0] = 0;
-        nc[1] = size;
-        nc[C * 3] = size;
-        nc[C * 3 - 1] = hop_num;
-    } else if (op_id % C == 0) {
-        nc[0] = nc[0] + nc[1];
-        nc[1] = nc[C * 2];
-        nc[C * 2] = 0;
-        nc[C * 2 + 1] = nc[0] + nc[1];
-        ec[0] = ec[0] + ec[1];
-        ec[1] = ec[2];
-        ec[2] = 0;
-        nc[C * 3 + op_id / C] = nc[0] + nc[1];
-        ec[C * 3 + op_id / C] = ec[1];
-        ec[C * 4 + op_id / C] = ec[0];
-    } else {
-        nc[(op_id % C) * 2] = nc[0];
-        nc[(op_id % C) * 2 + 1] = nc[1];
-    }
-}
-
 // ---- batch start -----------------------------------------------------------------------------
 
 // First kernel of every batch: empties the id map, zeroes the counters, stores the batch's parameters (the only
@@ -225,7 +199,11 @@ __global__ void batch_start_kernel(uint4 *slots2, int64_t n_pairs, int32_t *ctl,
         nc[threadIdx.x] = 0;  // cudaMemsetAsync of both counters, operator_impl.cu:158-159
         ec[threadIdx.x] = 0;
         __syncwarp(0xFFFFu);
-        if (threadIdx.x == 0) counter_update(nc, ec, 0, value.size, value.hop_num);
+        if (threadIdx.x == 0) {  // counter_update of op 0, operator_impl.cu:60-65
+            nc[1] = value.size;
+            nc[LEGION_INTRABATCH_CON * 3] = value.size;
+            nc[LEGION_INTRABATCH_CON * 3 - 1] = value.hop_num;
+        }
     }
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < value.size; idx += gridDim.x * blockDim.x) {
         const int64_t pos = value.first + idx;
