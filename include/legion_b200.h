@@ -297,7 +297,9 @@ int legion_batch_generate(void *stream, LegionFeatures *feature, LegionCache *ca
                           int32_t batch_size, int32_t counter, int32_t part_id, int32_t dev_id,
                           int32_t mode, int32_t is_presc, int32_t hop_num, int32_t dyn_cache);
 /* RandomSample, engine/operator_impl.cu:439-553: one hop (op_id = 3, 6, 9) of sampling,
- * dedup, relabel and counter bookkeeping; `count` is the fanout. */
+ * dedup, relabel and counter bookkeeping; `count` is the fanout.  The hop samples from every node known so far, so
+ * ops may be left out, repeated or issued in another order as long as nodes and edges fit the pool (device error 2 or 3
+ * otherwise); a hop that could then have more inputs than the pool's order gives it is sampled in parts. */
 int legion_random_sample(void *stream, LegionGraph *graph, LegionCache *cache, LegionPool *pool,
                          int32_t count, int32_t dev_id, int32_t op_id, int32_t is_presc, int32_t dyn_cache);
 /* FeatureCacheLookup, engine/operator_impl.cu:555-575: cache lookup + feature gather of the

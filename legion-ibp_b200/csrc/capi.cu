@@ -205,6 +205,7 @@ extern "C" int legion_pool_create_ahead(LegionPool **out, int32_t dev_id, int32_
             if (i < slots) e = cudaMalloc(&p->features[i], (size_t)(nodes * (int64_t)row_bytes_out));
             else p->features[i] = p->features[i % slots];
         }
+        p->hop_inputs[i] = batch_size;
         if (e == cudaSuccess) e = dmalloc(&p->labels[i], batch_size);
         if (e == cudaSuccess) e = dmalloc(&p->agg_src[i], pad_edges);
         if (e == cudaSuccess) e = dmalloc(&p->agg_dst[i], pad_edges);

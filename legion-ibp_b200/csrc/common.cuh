@@ -52,10 +52,13 @@ constexpr int32_t kEmptyVal = 0x7FFFFFFF;
 
 // ctl[] words (device scratch, one int32 each)
 enum Ctl {
-    // Both by the parity of the hop: hop h reads word h & 1 and leaves its result in the other, so that the CTA
-    // that learns the result may store it while others of the same launch still read.
+    // The first two are the result of a hop: its scan stores them, only the sampling kernel behind it reads them and
+    // leaves what the scan needs in the next three, so that neither kernel reads what a CTA of the same launch stores.
     CTL_N_NODES = 0,   // nodes known so far (== nc[0] + nc[1])
-    CTL_E_TOTAL = 2,   // edges of the hops already finished
+    CTL_E_TOTAL = 1,   // edges placed so far
+    CTL_HOP_N = 2,     // inputs of the hop in flight: the nodes known when it began
+    CTL_PART_N = 3,    // nodes and edges before the launches in flight (a hop is one pair of launches, or several:
+    CTL_PART_E = 6,    //   launch_sample_hop)
     CTL_TILE = 4,      // next tile of the scan over the hop's entries
     CTL_SEEDS_IN = 5,  // the seeds have entered the id map (with the batch's first hop)
     CTL_ERROR = 7,     // first error raised by a kernel (0 = none)
@@ -194,6 +197,7 @@ struct LegionPool {
     int32_t row_bytes_out;
     int32_t pipes;
     int64_t max_nodes, max_edges, max_hop_edges;
+    int64_t hop_inputs[LEGION_MAX_PIPES];  // most nodes that the batch on the pipe can know after the ops issued so far
     int64_t feat_rows;
     // Hand-off buffers, `slots` sets: what a consumer reads (the seven buffers that are published to trainers).
     // With slots == pipes they ARE the pipes' own output buffers below.  With fewer slots than pipes

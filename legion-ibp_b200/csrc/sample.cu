@@ -230,6 +230,12 @@ __global__ void batch_start_kernel(uint4 *slots2, int64_t n_pairs, int32_t *ctl,
 
 // ---- one hop -----------------------------------------------------------------------------------
 
+// A stretch of a hop's inputs (launch_sample_hop).
+struct HopPart {
+    int32_t first, count, last;
+};
+__device__ __forceinline__ int part_inputs(const HopPart &p, int inputs) { return max(0, min(p.count, inputs - p.first)); }
+
 // Lanes that share an input node: the fanout, rounded up to 8, 16 or 32.
 static inline int group_lanes(int fanout) { return fanout <= 8 ? 8 : fanout <= 16 ? 16 : 32; }
 
@@ -239,23 +245,31 @@ static inline int group_lanes(int fanout) { return fanout <= 8 ? 8 : fanout <= 1
 // Bound by latency: neighbour id from HBM, map slot and compare-and-swap in L2, one after the other; small chunks
 // keep every warp of the chip on its own chain.
 // In the batch's first hop the seeds enter the map too, each with its position.
-template <int G>
+// PART: the launch takes the inputs [part.first, part.first + part.count) of the hop.
+template <int G, bool PART>
 __global__ void __launch_bounds__(256, 6)
 hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict__ indices, const int32_t *ids,
                   int32_t fanout, uint32_t hop, const BatchCtl *__restrict__ b, int2 *rec, MapSlot *map, MapDims mask,
-                  int32_t *ctl, const int32_t *nc, uint8_t *edge_cnt, uint32_t *tile_state, int64_t max_entries)
+                  int32_t *ctl, const int32_t *nc, uint8_t *edge_cnt, uint32_t *tile_state, int64_t max_entries, HopPart part)
 {
     pdl_wait();
     pdl_trigger();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, n_threads = gridDim.x * blockDim.x;
     const int late = ctl[CTL_LATE_ERROR];
+    const int known = ctl[CTL_N_NODES];
+    const int inputs = !PART || part.first == 0 ? known : ctl[CTL_HOP_N];
     if (tid == 0) {
         ctl[CTL_TILE] = 0;
+        if (!PART || part.first == 0) ctl[CTL_HOP_N] = known;
+        ctl[CTL_PART_N] = known;
+        ctl[CTL_PART_E] = ctl[CTL_E_TOTAL];
         if (late != DERR_NONE) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, late);
     }
     if (ctl[CTL_ERROR] != DERR_NONE || late != DERR_NONE) return;
-    const int n = ctl[CTL_N_NODES + (hop & 1)];
-    if ((int64_t)n * fanout > max_entries) {  // a hop out of the pool's order: more inputs than this fanout was sized for
+    const int lo = PART ? part.first : 0;
+    const int n = PART && !part.last ? part_inputs(part, inputs) : inputs - lo;
+    // (cannot happen unless a captured sequence of ops is replayed behind others than it was captured behind)
+    if (n > 0 && (int64_t)n * fanout > max_entries) {
         if (threadIdx.x == 0) atomicCAS(&ctl[CTL_ERROR], DERR_NONE, DERR_EDGE_OVERFLOW);
         return;
     }
@@ -281,7 +295,7 @@ hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict_
         int64_t my_start = 0;
         int32_t my_deg = 0;
         if (lane < here) {
-            const int32_t id = __ldcg(&ids[first + lane]);
+            const int32_t id = __ldcg(&ids[lo + first + lane]);
             if (id >= 0) {
                 if (id < n_limit) {
                     my_start = __ldg(&indptr[id]);
@@ -290,19 +304,19 @@ hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict_
                     ctl[CTL_BAD_IDS] = 1;
                 }
             }
-            edge_cnt[cnt0 + first + lane] = (uint8_t)min((uint32_t)my_deg, k);
-            if (!seeds_in && id >= 0) map_insert_min(map, mask, id, (int)first + lane, ctl);
+            edge_cnt[cnt0 + lo + first + lane] = (uint8_t)min((uint32_t)my_deg, k);
+            if (!seeds_in && id >= 0) map_insert_min(map, mask, id, lo + (int)first + lane, ctl);
         }
         for (int j0 = 0; j0 < here; j0 += NPW) {
             const int j = j0 + lane / G;
             const int64_t start = __shfl_sync(kFull, (long long)my_start, j & 31);
             const uint32_t deg_j = (uint32_t)__shfl_sync(kFull, my_deg, j & 31);
             const uint32_t deg = j < here ? deg_j : 0u;
-            const uint32_t i = (uint32_t)first + (uint32_t)j;
+            const uint32_t i = (uint32_t)first + (uint32_t)j;  // of this launch's inputs
             // drawn: deg >= 2k draws the k positions to take, k < deg < 2k the deg - k positions to leave out
             const bool leave_out = deg > k && deg < 2 * k;
             const int m = deg <= k ? 0 : leave_out ? (int)(deg - k) : (int)k;
-            const uint32_t x = draw_distinct<G>(m, deg, i, hop, batch_id, k0, k1, max_rounds, lane);
+            const uint32_t x = draw_distinct<G>(m, deg, (uint32_t)lo + i, hop, batch_id, k0, k1, max_rounds, lane);
             int out_slot = -1, out_slot2 = -1;   // slot of this lane's first edge, second edge in out_slot2
             uint32_t pos = sub, pos2 = sub + G;
             if (!leave_out) {
@@ -348,9 +362,10 @@ constexpr uint32_t kTileCounted = 0x80000000u;
 // The end of a hop that found c nodes and e edges: counter_update for op_id (a multiple of LEGION_INTRABATCH_CON) on
 // both counter arrays, held one word per lane by the warp that calls; with a mirror (the last hop) both arrays also go
 // to page-locked host memory, one posted store per lane: the host learns the sizes of the batch without a copy-engine
-// transfer queued behind other batches' exports.
+// transfer queued behind other batches' exports.  The end of a part that is not the hop's last (`closes` false) only
+// adds to the words that count the hop.
 __device__ __forceinline__ void advance_counters(int word, int c, int e, int n0, int e_base, int op_id, int32_t *ctl, int32_t *nc,
-                                                 int32_t *ec, int32_t *mirror)
+                                                 int32_t *ec, int32_t *mirror, bool closes)
 {
     constexpr int C = LEGION_INTRABATCH_CON;
     const int lane = threadIdx.x & 31, h = op_id / C;
@@ -359,7 +374,11 @@ __device__ __forceinline__ void advance_counters(int word, int c, int e, int n0,
     const int done = __shfl_sync(kFull, word, 16) + __shfl_sync(kFull, word, 17);
     const int drawn = __shfl_sync(kFull, word, 18) + e;                                     // operator_impl.cu:282
     bool changed = true;                                                                    // operator_impl.cu:66-80
-    if (lane == 0) word = known;
+    if (!closes) {
+        if (lane == C * 2) nc[C * 2] = found;
+        if (lane == 16 + 2) ec[2] = drawn;
+        changed = false;
+    } else if (lane == 0) word = known;
     else if (lane == 1) word = found;
     else if (lane == C * 2 || lane == 16 + 2) word = 0;
     else if (lane == C * 2 + 1 || lane == C * 3 + h) word = known + found;
@@ -370,9 +389,8 @@ __device__ __forceinline__ void advance_counters(int word, int c, int e, int n0,
     if (changed) *(lane < 16 ? nc + lane : ec + (lane - 16)) = word;
     if (mirror != nullptr) mirror[lane] = word;
     if (lane == 0) {
-        const int next = h & 1;  // the parity of the hop that follows
-        ctl[CTL_N_NODES + next] = n0 + c;
-        ctl[CTL_E_TOTAL + next] = e_base + e;
+        ctl[CTL_N_NODES] = n0 + c;
+        ctl[CTL_E_TOTAL] = e_base + e;
         ctl[CTL_SEEDS_IN] = 1;
     }
 }
@@ -391,10 +409,11 @@ __device__ __forceinline__ void advance_counters(int word, int c, int e, int n0,
 // Bound by L2 latency: record, map slot, counts, map slot.  Four entries per thread: four map reads in flight and fewer
 // counts to add up.  (Tiles of 256 in small hops, for more CTAs: eight batches of 800 seeds, [25,10], 267 against 264 us,
 // and 295 where hop 2 used them too; one batch alone the same.)
+template <bool PART>
 __global__ void __launch_bounds__(kScanThreads, 6)
 hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_state, int32_t *ids, MapSlot *map,
                   int32_t *src_global, int32_t *agg_src, int32_t *agg_dst, int32_t *ctl, int32_t *nc, int32_t *ec, int op_id,
-                  const BatchCtl *__restrict__ b, int last_hop, int64_t max_nodes, int64_t max_edges)
+                  const BatchCtl *__restrict__ b, int last_hop, int64_t max_nodes, int64_t max_edges, HopPart part)
 {
     pdl_wait();
     pdl_trigger();
@@ -404,18 +423,19 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
     __shared__ int s_edges[kScanThreads / 32], s_new[kScanThreads / 32];
     __shared__ int s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(&ctl[CTL_TILE], 1);
-    const int hop = op_id / LEGION_INTRABATCH_CON - 1;
-    const int n0 = ctl[CTL_N_NODES + (hop & 1)];
-    const int e_base = ctl[CTL_E_TOTAL + (hop & 1)];
+    const int n0 = ctl[CTL_PART_N];
+    const int e_base = ctl[CTL_PART_E];
+    const int inputs = PART ? part_inputs(part, ctl[CTL_HOP_N]) : n0;
+    const bool closes = !PART || part.last;
     const bool ok = ctl[CTL_ERROR] == DERR_NONE;  // raised before this kernel: nobody raises it while it runs
     // both counter arrays, one word per lane of the first warp (only this kernel changes what it uses of them)
     const int counter = threadIdx.x < 16 ? nc[threadIdx.x] : threadIdx.x < 32 ? ec[threadIdx.x - 16] : 0;
-    int32_t *const mirror = last_hop ? b->mirror : nullptr;
-    const int total = ok ? n0 * fanout : 0;
+    int32_t *const mirror = last_hop && closes ? b->mirror : nullptr;
+    const int total = ok ? inputs * fanout : 0;
     const int n_tiles = (total + TILE - 1) / TILE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int next = 0, edges = 0, fresh = 0;  // tiles before `next` hold `edges` edges and `fresh` new nodes
-    if (n_tiles == 0 && blockIdx.x == 0 && warp == 0) advance_counters(counter, 0, 0, n0, e_base, op_id, ctl, nc, ec, mirror);
+    if (n_tiles == 0 && blockIdx.x == 0 && warp == 0) advance_counters(counter, 0, 0, n0, e_base, op_id, ctl, nc, ec, mirror, closes);
     for (;;) {
         __syncthreads();
         const int tile = s_tile;
@@ -465,10 +485,11 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
             break;
         }
         if (tile == n_tiles - 1 && warp == 0)
-            advance_counters(counter, fresh + tile_new, edges + tile_edges, n0, e_base, op_id, ctl, nc, ec, mirror);
+            advance_counters(counter, fresh + tile_new, edges + tile_edges, n0, e_base, op_id, ctl, nc, ec, mirror, closes);
         int at = e_base + edges + (mine & 0xFFFF);
         int local = n0 + fresh + (mine >> 16);
         int dst = base / fanout, in_row = base - dst * fanout;
+        if (PART) dst += part.first;
         int where[IPT];
 #pragma unroll
         for (int j = 0; j < IPT; ++j) {
@@ -576,6 +597,7 @@ BatchCtl make_batch_ctl(const LegionPool *p, const LegionCache *c, const int32_t
 int launch_batch_generate(cudaStream_t s, LegionPool *p, const BatchCtl &v)
 {
     const int pipe = p->pipe;
+    p->hop_inputs[pipe] = p->batch_size;
     const int64_t n_pairs = ((int64_t)p->map_front_mask + 1) / 2;
     const int64_t back_pairs = ((int64_t)p->map_mask + 1) / 2;
     // sized for the front region and the seeds; when the back region has to be cleared too, the CTAs loop longer
@@ -587,37 +609,51 @@ int launch_batch_generate(cudaStream_t s, LegionPool *p, const BatchCtl &v)
     return LEGION_OK;
 }
 
-template <int G>
+template <int G, bool PART>
 static cudaError_t launch_hop_sample(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop,
-                                     int64_t inputs)
+                                     int64_t inputs, HopPart part)
 {
     const int pipe = p->pipe;
-    return launch_dep(p, hop_sample_kernel<G>, grid_for(inputs, 8 * (32 / G), p->sm_count * 6), 256, s, g->indptr, g->indices, p->ids[pipe], fanout,
+    return launch_dep(p, hop_sample_kernel<G, PART>, grid_for(inputs, 8 * (32 / G), p->sm_count * 6), 256, s, g->indptr, g->indices, p->ids[pipe], fanout,
                       (uint32_t)hop, p->bctl[pipe], p->edge_rec[pipe], p->map[pipe], MapDims{ p->map_front_mask, p->map_mask },
-                      p->ctl[pipe], p->node_counter[pipe], p->edge_cnt[pipe], p->tile_state[pipe], p->max_hop_edges);
+                      p->ctl[pipe], p->node_counter[pipe], p->edge_cnt[pipe], p->tile_state[pipe], p->max_hop_edges, part);
 }
 
-static cudaError_t launch_hop_finish(cudaStream_t s, LegionPool *p, int32_t fanout, int32_t hop, int32_t op_id, int64_t edges)
+template <bool PART>
+static int launch_hop_pair(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop, int32_t op_id,
+                           int64_t inputs, HopPart part)
 {
     const int pipe = p->pipe;
-    return launch_dep(p, hop_finish_kernel, grid_for(edges, kTile, p->sm_count * 8), kScanThreads, s, p->edge_rec[pipe],
-                      fanout, p->tile_state[pipe], p->ids[pipe], p->map[pipe], p->src_global[pipe], p->agg_src[pipe],
-                      p->agg_dst[pipe], p->ctl[pipe], p->node_counter[pipe], p->edge_counter[pipe], op_id, p->bctl[pipe],
-                      hop + 1 == p->hop_num ? 1 : 0, p->max_nodes, p->max_edges);
+    switch (group_lanes(fanout)) {
+    case 8: LG_CUDA((launch_hop_sample<8, PART>(s, p, g, fanout, hop, inputs, part))); break;
+    case 16: LG_CUDA((launch_hop_sample<16, PART>(s, p, g, fanout, hop, inputs, part))); break;
+    default: LG_CUDA((launch_hop_sample<32, PART>(s, p, g, fanout, hop, inputs, part))); break;
+    }
+    LG_CUDA(launch_dep(p, hop_finish_kernel<PART>, grid_for(inputs * fanout, kTile, p->sm_count * 8), kScanThreads, s, p->edge_rec[pipe],
+                       fanout, p->tile_state[pipe], p->ids[pipe], p->map[pipe], p->src_global[pipe], p->agg_src[pipe],
+                       p->agg_dst[pipe], p->ctl[pipe], p->node_counter[pipe], p->edge_counter[pipe], op_id, p->bctl[pipe],
+                       hop + 1 == p->hop_num ? 1 : 0, p->max_nodes, p->max_edges, part));
+    return LEGION_OK;
 }
 
+// In the pool's order every hop's entries (inputs * fanout) fit the records, which legion_pool_create sizes for that.  The
+// ops may also come in another order, or more than once; a hop that then could have more inputs is sampled in parts of
+// as many as fit, one pair of launches each.  The nodes of an earlier part have their local ids when a later one meets
+// them, so the result is that of one pair over all inputs.
 int launch_sample_hop(cudaStream_t s, LegionPool *p, const LegionGraph *g, int32_t fanout, int32_t hop, int32_t op_id)
 {
-    // worst-case sizes of this hop: inputs = all nodes so far, edges = inputs * fanout
     int64_t inputs = p->batch_size;
-    for (int h = 0; h < hop; ++h) inputs += inputs * p->fanout[h];
-    const int64_t edges = inputs * fanout;
-    switch (group_lanes(fanout)) {
-    case 8: LG_CUDA(launch_hop_sample<8>(s, p, g, fanout, hop, inputs)); break;
-    case 16: LG_CUDA(launch_hop_sample<16>(s, p, g, fanout, hop, inputs)); break;
-    default: LG_CUDA(launch_hop_sample<32>(s, p, g, fanout, hop, inputs)); break;
+    for (int h = 0; h < hop; ++h) inputs += inputs * p->fanout[h];  // in the pool's order
+    if (inputs < p->hop_inputs[p->pipe]) inputs = p->hop_inputs[p->pipe];
+    const int64_t known = inputs + inputs * fanout;
+    p->hop_inputs[p->pipe] = known < p->max_nodes ? known : p->max_nodes;
+    if (inputs * fanout <= p->max_hop_edges) return launch_hop_pair<false>(s, p, g, fanout, hop, op_id, inputs, HopPart{ 0, 0, 1 });
+    const int64_t fit = p->max_hop_edges / fanout;
+    for (int64_t first = 0; first < inputs; first += fit) {
+        const int rc = launch_hop_pair<true>(s, p, g, fanout, hop, op_id, fit,
+                                             HopPart{ (int32_t)first, (int32_t)fit, first + fit >= inputs ? 1 : 0 });
+        if (rc != LEGION_OK) return rc;
     }
-    LG_CUDA(launch_hop_finish(s, p, fanout, hop, op_id, edges));
     return LEGION_OK;
 }
 

@@ -288,3 +288,70 @@ def test_large_hop_matches_host_replay(oracle_mod):
         _compare(_fetch(pool), oracle_mod.run_batch(indptr, indices, train, labels, 9000, 0, [25, 16], it, 13))
         assert pool.device_error() == 0
     pool.close(); f.close(); g.close()
+
+
+def _replay_ops(O, indptr, indices, seeds, fanout, ops, global_batch, seed):
+    """Host replay of the sampling ops in any order: every op samples all nodes known so far with the fanout and the RNG
+    word of its hop; edges follow one another, new nodes are numbered in order of first appearance."""
+    nc, ec = np.zeros(16, np.int32), np.zeros(16, np.int32)
+    ids = list(seeds)
+    local = {}
+    for i, u in enumerate(ids):
+        local.setdefault(int(u), i)
+    O.counter_update(nc, ec, 0, len(ids), len(fanout))
+    src, dst, src_global = [], [], []
+    for op in ops:
+        h = op // 3 - 1
+        s, d = O.sample_hop(indptr, indices, np.array(ids, np.int32), fanout[h], h, global_batch, seed)
+        before = len(ids)
+        for u in s:
+            if int(u) not in local:
+                local[int(u)] = len(ids)
+                ids.append(int(u))
+            src.append(local[int(u)])
+        src_global += list(s)
+        dst += list(d)
+        nc[6] += len(ids) - before
+        ec[2] += len(s)
+        O.counter_update(nc, ec, op, 0, 0)
+    return dict(node_counter=nc, edge_counter=ec, ids=ids, agg_src=src, agg_dst=dst, src_global=src_global)
+
+
+def _fetch_known(pool, pipe=0):
+    """What the ops so far have left, whichever they were."""
+    nc = pool.read(L.BUF_NODE_COUNTER, pipe, 16, np.int32)
+    ec = pool.read(L.BUF_EDGE_COUNTER, pipe, 16, np.int32)
+    n, e = int(nc[0] + nc[1]), int(ec[0] + ec[1])
+    return dict(node_counter=nc, edge_counter=ec, ids=pool.read(L.BUF_IDS, pipe, n, np.int32),
+                agg_src=pool.read(L.BUF_AGG_SRC, pipe, e, np.int32), agg_dst=pool.read(L.BUF_AGG_DST, pipe, e, np.int32),
+                src_global=pool.read(L.BUF_SRC_GLOBAL, pipe, e, np.int32))
+
+
+@pytest.mark.parametrize("fanout,ops", [([25, 10], [6]), ([25, 10], [6, 3]), ([10, 25], [6, 3]), ([25, 10], [3, 3]),
+                                        ([25, 10], [3, 3, 6]), ([25, 10], [6, 6, 3]), ([5, 15, 10], [3, 9]),
+                                        ([5, 15, 10], [9, 6, 3]), ([16, 2], [6, 6, 3]), ([30, 1], [6, 6, 6, 3, 6])])
+@pytest.mark.parametrize("pipes", [1, 2])
+def test_sampling_ops_in_any_order(oracle_mod, fanout, ops, pipes):
+    """Ops that skip a hop, come in another order or more than once, as long as their nodes and edges fit the pool; the
+    repeated ones have more inputs than the records hold entries for and are sampled in parts."""
+    n_nodes, batch = 20000, 40
+    indptr, indices = small_graph(n_nodes, 30000, 51)
+    train = np.random.default_rng(2).permutation(n_nodes)[:batch * 3].astype(np.int32)
+    train[5] = train[7]
+    g, f, pool = _setup(indptr, indices, train, train.copy(), batch, fanout, pipes=pipes)
+    pool.set_rng(21, 64)
+    for it in range(3):
+        pool.set_batch(it, L.TRAINMODE, it % pipes, it)
+        L.BatchGenerate(None, f, None, pool, batch, it, 0, 0, L.TRAINMODE, False, len(fanout))
+        for op in ops:
+            L.RandomSample(None, g, None, pool, fanout[op // 3 - 1], 0, op)
+        want = _replay_ops(oracle_mod, indptr, indices, train[it * batch:(it + 1) * batch], fanout, ops, it, 21)
+        got = _fetch_known(pool, it % pipes)
+        assert len(want["ids"]) <= pool.max_nodes and len(want["agg_src"]) <= pool.max_edges
+        for k in want:
+            np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+        assert pool.device_error() == 0
+    # the pool's own order afterwards
+    _run_ops(g, f, pool, batch, 0, fanout, global_batch=9)
+    _compare(_fetch(pool), oracle_mod.run_batch(indptr, indices, train, train, batch, 0, fanout, 9, 21))
+    pool.close(); f.close(); g.close()
