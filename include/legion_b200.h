@@ -74,6 +74,8 @@ int legion_set_tunable(const char *name, int32_t value);
  * variable LEGION_GATHER_ENGINE); "pdl" 1 = the sampling kernels of a batch are launched as programmatic
  * dependents of one another in every pool (start value from LEGION_PDL; applies to runners created afterwards), 0 = only
  * in pools of one pipe or at most 65,536 nodes;
+ * "scan_wait_limit": reads of a wait inside the scan of a hop before it gives up (default 2^20, about a second; 0 and, for
+ * waits that give up whatever they read, -1 are for tests; applies to ops issued and runners created afterwards);
  * "map_front_shift" s: the front region of a pool's id map gets 1 / 2^s of the worst-case slots
  * (-1, the default: an eighth, but at least 2^20 slots where the worst case has that many; pools
  * created afterwards). */
@@ -283,7 +285,9 @@ int legion_pool_set_rng(LegionPool *p, uint64_t seed, int32_t max_rounds);
 /* First error raised on the device since the last reset (the reference prints and exits,
  * engine/operator_impl.cu:17-25): 0 none, 1 id map full, 2 edge buffer overflow, 3 node buffer
  * overflow, 4 a bulk copy of the gather timed out (the pipe's output is invalid; stop issuing on it),
- * 6 a wait inside the scan of a hop did not end within its limit (the batch ends with the hops before it);
+ * 6 a wait inside the scan of a hop did not end within its limit.  After 1, 2, 3 and 6 the counters are those of the hops
+ * before (after 6 they may include the hop: its indices are then in range, but some name node 0); the batch is to be discarded, the next one
+ * on the pipe is sampled once the error has been reset;
  * 5 a seed id (or a neighbour id stored in the topology) outside [0, n_nodes) was met: such an id is
  * never used as an index, its slot in the batch reads -1 like a slot past the end of the seed list
  * (engine/operator_impl.cu:41-43), and the rest of the batch is complete.  Synchronises `stream`. */

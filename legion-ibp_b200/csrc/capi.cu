@@ -323,7 +323,7 @@ extern "C" int legion_pool_set_rng(LegionPool *p, uint64_t seed, int32_t max_rou
 
 // First error raised by a kernel of this pool since the last reset (0 = none): 1 id map full,
 // 2 edge buffer overflow, 3 node buffer overflow, 4 bulk copy timed out, 6 a wait of the hop's scan timed out (these
-// stop the batch);
+// stop the batch, whose counters then end with the hops before);
 // 5 a seed or neighbour id outside [0, n_nodes) was met: it was skipped without being read, the
 // rest of the batch is complete.  Synchronises the stream.
 extern "C" int legion_pool_device_error(LegionPool *p, void *stream, int32_t *err, int32_t reset)

@@ -252,6 +252,7 @@ namespace legion {
 // kernel launchers (defined in sample.cu / gather.cu / cache.cu)
 extern int g_pdl;
 extern int g_map_front_shift;
+extern int g_scan_wait_limit;
 int launch_batch_generate(cudaStream_t s, LegionPool *p, const BatchCtl &ctl);
 BatchCtl make_batch_ctl(const LegionPool *p, const LegionCache *c, const int32_t *all_ids, const int32_t *all_labels,
                         int32_t total_cap, int64_t first, int32_t size, int64_t n_nodes);

@@ -1516,6 +1516,11 @@ extern "C" int legion_set_tunable(const char *name, int32_t value)
         g_pdl = value;  // takes effect for runners created (graphs captured) afterwards
         return LEGION_OK;
     }
+    if (strcmp(name, "scan_wait_limit") == 0) {
+        LG_ARG(value >= -1 && value <= 1 << 30, "scan_wait_limit must be -1 .. 2^30");
+        g_scan_wait_limit = value;  // ops issued and graphs captured afterwards
+        return LEGION_OK;
+    }
     if (strcmp(name, "gather_engine") == 0) {
         LG_ARG(value == 0 || value == 1, "gather_engine must be 0 (registers) or 1 (bulk copies)");
         g_gather_engine = value;

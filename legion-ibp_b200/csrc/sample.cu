@@ -356,23 +356,25 @@ hop_sample_kernel(const int64_t *__restrict__ indptr, const int32_t *__restrict_
     }
 }
 
-constexpr int kScanWaitLimit = 1 << 20;
 constexpr uint32_t kTileCounted = 0x80000000u;
+// reads of a wait inside the scan before it gives up (legion_set_tunable "scan_wait_limit"); about a second
+constexpr int kScanWaitLimit = 1 << 20;
+int g_scan_wait_limit = kScanWaitLimit;
 
 // The end of a hop that found c nodes and e edges: counter_update for op_id (a multiple of LEGION_INTRABATCH_CON) on
 // both counter arrays, held one word per lane by the warp that calls; with a mirror (the last hop) both arrays also go
 // to page-locked host memory, one posted store per lane: the host learns the sizes of the batch without a copy-engine
 // transfer queued behind other batches' exports.  The end of a part that is not the hop's last (`closes` false) only
-// adds to the words that count the hop.
+// adds to the words that count the hop.  A hop that failed has found nothing: the batch ends with the hops before it.
 __device__ __forceinline__ void advance_counters(int word, int c, int e, int n0, int e_base, int op_id, int32_t *ctl, int32_t *nc,
-                                                 int32_t *ec, int32_t *mirror, bool closes)
+                                                 int32_t *ec, int32_t *mirror, bool closes, bool failed)
 {
     constexpr int C = LEGION_INTRABATCH_CON;
     const int lane = threadIdx.x & 31, h = op_id / C;
     const int known = __shfl_sync(kFull, word, 0) + __shfl_sync(kFull, word, 1);
-    const int found = __shfl_sync(kFull, word, C * 2) + c;                                  // operator_impl.cu:281
+    const int found = failed ? 0 : __shfl_sync(kFull, word, C * 2) + c;                     // operator_impl.cu:281
     const int done = __shfl_sync(kFull, word, 16) + __shfl_sync(kFull, word, 17);
-    const int drawn = __shfl_sync(kFull, word, 18) + e;                                     // operator_impl.cu:282
+    const int drawn = failed ? 0 : __shfl_sync(kFull, word, 18) + e;                        // operator_impl.cu:282
     bool changed = true;                                                                    // operator_impl.cu:66-80
     if (!closes) {
         if (lane == C * 2) nc[C * 2] = found;
@@ -400,7 +402,8 @@ __device__ __forceinline__ void advance_counters(int word, int c, int e, int n0,
 // one word per tile, so nothing is passed from tile to tile) and places its edges and new nodes.
 // Tiles are handed out in order by a ticket and a CTA publishes its counts before it waits for others, so the
 // lowest unfinished tile never waits: whatever else shares the GPU, every wait ends.  All waits are bounded
-// (DERR_SCAN_TIMEOUT).
+// (DERR_SCAN_TIMEOUT).  A CTA that gives up, or whose edges do not fit, places nothing more but still hands out and
+// counts tiles, so that the CTA of the last tile always closes the hop.
 // The CTA of the last tile knows the hop's totals as soon as it has added up the others' and advances the counters
 // there and then: no CTA waits for the end of all others (the two that did, one of them behind a fence over the stores
 // of the whole CTA, were 4 of the 9-11 us that the launch took on two tiles).
@@ -413,7 +416,8 @@ template <bool PART>
 __global__ void __launch_bounds__(kScanThreads, 6)
 hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_state, int32_t *ids, MapSlot *map,
                   int32_t *src_global, int32_t *agg_src, int32_t *agg_dst, int32_t *ctl, int32_t *nc, int32_t *ec, int op_id,
-                  const BatchCtl *__restrict__ b, int last_hop, int64_t max_nodes, int64_t max_edges, HopPart part)
+                  const BatchCtl *__restrict__ b, int last_hop, int64_t max_nodes, int64_t max_edges, HopPart part,
+                  int wait_limit)
 {
     pdl_wait();
     pdl_trigger();
@@ -435,7 +439,9 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
     const int n_tiles = (total + TILE - 1) / TILE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int next = 0, edges = 0, fresh = 0;  // tiles before `next` hold `edges` edges and `fresh` new nodes
-    if (n_tiles == 0 && blockIdx.x == 0 && warp == 0) advance_counters(counter, 0, 0, n0, e_base, op_id, ctl, nc, ec, mirror, closes);
+    int failed = DERR_NONE;
+    if (n_tiles == 0 && blockIdx.x == 0 && warp == 0)
+        advance_counters(counter, 0, 0, n0, e_base, op_id, ctl, nc, ec, mirror, closes, !ok);
     for (;;) {
         __syncthreads();
         const int tile = s_tile;
@@ -459,62 +465,76 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
         int mine = block_excl_scan(count, &tile_count, smem);
         if (threadIdx.x == 0) *(volatile uint32_t *)&tile_state[tile] = kTileCounted | (uint32_t)tile_count;
         int se = 0, sn = 0;
-        bool late = false;
-        for (int q = next + threadIdx.x; q < tile; q += kScanThreads) {
+        bool late = failed != DERR_NONE;
+        for (int q = next + threadIdx.x; q < tile && !late; q += kScanThreads) {
             uint32_t w = __ldcg(&tile_state[q]);
-            for (int spin = 0; (w & kTileCounted) == 0u && spin < kScanWaitLimit; ++spin) w = *(volatile uint32_t *)&tile_state[q];
-            late |= (w & kTileCounted) == 0u;
+            for (int spin = 0; (w & kTileCounted) == 0u && spin < wait_limit; ++spin) w = *(volatile uint32_t *)&tile_state[q];
+            if ((w & kTileCounted) == 0u) {
+                // said before it is settled: the CTA of the last tile, should it have seen this count, then sees the word
+                atomicCAS(&ctl[CTL_LATE_ERROR], DERR_NONE, DERR_SCAN_TIMEOUT);
+                __threadfence();
+                w = *(volatile uint32_t *)&tile_state[q];
+            }
+            late = (w & kTileCounted) == 0u || wait_limit < 0;
             se += (int)(w & 0xFFFFu);
             sn += (int)((w & ~kTileCounted) >> 16);
         }
         se = __reduce_add_sync(kFull, se);
         sn = __reduce_add_sync(kFull, sn);
         if (lane == 0) { s_edges[warp] = se; s_new[warp] = sn; }
-        if (__syncthreads_or(late ? 1 : 0)) {
-            if (threadIdx.x == 0) ctl[CTL_LATE_ERROR] = DERR_SCAN_TIMEOUT;
-            break;
-        }
+        if (__syncthreads_or(late ? 1 : 0) && failed == DERR_NONE) failed = DERR_SCAN_TIMEOUT;
 #pragma unroll
         for (int w = 0; w < kScanThreads / 32; ++w) { edges += s_edges[w]; fresh += s_new[w]; }
         const int tile_edges = tile_count & 0xFFFF, tile_new = tile_count >> 16;
         // (cannot happen with the buffers that legion_pool_create sizes for this fanout)
-        const bool fits = (int64_t)e_base + edges + tile_edges <= max_edges && (int64_t)n0 + fresh + tile_new <= max_nodes;
-        if (!fits) {
-            if (threadIdx.x == 0)
-                ctl[CTL_LATE_ERROR] = (int64_t)e_base + edges + tile_edges > max_edges ? DERR_EDGE_OVERFLOW : DERR_NODE_OVERFLOW;
-            break;
-        }
+        if (failed == DERR_NONE && (int64_t)e_base + edges + tile_edges > max_edges) failed = DERR_EDGE_OVERFLOW;
+        if (failed == DERR_NONE && (int64_t)n0 + fresh + tile_new > max_nodes) failed = DERR_NODE_OVERFLOW;
+        if (failed != DERR_NONE && threadIdx.x == 0) atomicCAS(&ctl[CTL_LATE_ERROR], DERR_NONE, failed);
         if (tile == n_tiles - 1 && warp == 0)
-            advance_counters(counter, fresh + tile_new, edges + tile_edges, n0, e_base, op_id, ctl, nc, ec, mirror, closes);
-        int at = e_base + edges + (mine & 0xFFFF);
-        int local = n0 + fresh + (mine >> 16);
-        int dst = base / fanout, in_row = base - dst * fanout;
-        if (PART) dst += part.first;
-        int where[IPT];
+            advance_counters(counter, fresh + tile_new, edges + tile_edges, n0, e_base, op_id, ctl, nc, ec, mirror, closes,
+                             failed != DERR_NONE);
+        if (failed == DERR_NONE) {
+            int at = e_base + edges + (mine & 0xFFFF);
+            int local = n0 + fresh + (mine >> 16);
+            int dst = base / fanout, in_row = base - dst * fanout;
+            if (PART) dst += part.first;
+            int where[IPT];
 #pragma unroll
-        for (int j = 0; j < IPT; ++j) {
-            where[j] = -1;
-            if (slot[j] >= 0) {
-                src_global[at] = u[j];
-                agg_dst[at] = dst;
-                if (val[j] == kNewBase + base + j) {
-                    ids[local] = u[j];
-                    __stcg(&map[slot[j]].val, local);
-                    val[j] = local++;
+            for (int j = 0; j < IPT; ++j) {
+                where[j] = -1;
+                if (slot[j] >= 0) {
+                    src_global[at] = u[j];
+                    agg_dst[at] = dst;
+                    if (val[j] == kNewBase + base + j) {
+                        ids[local] = u[j];
+                        __stcg(&map[slot[j]].val, local);
+                        val[j] = local++;
+                    }
+                    if (val[j] < kNewBase) agg_src[at] = val[j];
+                    else where[j] = at;  // first reached by another entry of this hop
+                    ++at;
                 }
-                if (val[j] < kNewBase) agg_src[at] = val[j];
-                else where[j] = at;  // first reached by another entry of this hop
-                ++at;
+                if (++in_row == fanout) { in_row = 0; ++dst; }
             }
-            if (++in_row == fanout) { in_row = 0; ++dst; }
-        }
+            const bool last_tile = tile == n_tiles - 1 && warp == 0;
+            const int others = last_tile ? *(volatile int32_t *)&ctl[CTL_LATE_ERROR] : DERR_NONE;
 #pragma unroll
-        for (int j = 0; j < IPT; ++j) {
-            if (where[j] < 0) continue;
-            int v = __ldcg(&map[slot[j]].val);
-            for (int spin = 0; v >= kNewBase && spin < kScanWaitLimit; ++spin) v = *(volatile int32_t *)&map[slot[j]].val;
-            if (v >= kNewBase) ctl[CTL_LATE_ERROR] = DERR_SCAN_TIMEOUT;
-            agg_src[where[j]] = v;
+            for (int j = 0; j < IPT; ++j) {
+                if (where[j] < 0) continue;
+                int v = __ldcg(&map[slot[j]].val);
+                for (int spin = 0; v >= kNewBase && spin < wait_limit; ++spin) {
+                    v = *(volatile int32_t *)&map[slot[j]].val;
+                    if ((spin & 1023) == 1023 && *(volatile int32_t *)&ctl[CTL_LATE_ERROR] != DERR_NONE) break;
+                }
+                if (v >= kNewBase) {
+                    atomicCAS(&ctl[CTL_LATE_ERROR], DERR_NONE, DERR_SCAN_TIMEOUT);
+                    v = 0;  // a local id all the same: the batch is reported, not left with an index that is none
+                }
+                agg_src[where[j]] = v;
+            }
+            // a CTA that gave up while this one did not: the hop is closed once more, without what it found
+            if (last_tile && __any_sync(kFull, others != DERR_NONE))
+                advance_counters(counter, 0, 0, n0, e_base, op_id, ctl, nc, ec, mirror, closes, true);
         }
         if (n_tiles <= (int)gridDim.x) break;  // a tile for every CTA
         edges += tile_edges;
@@ -632,7 +652,7 @@ static int launch_hop_pair(cudaStream_t s, LegionPool *p, const LegionGraph *g, 
     LG_CUDA(launch_dep(p, hop_finish_kernel<PART>, grid_for(inputs * fanout, kTile, p->sm_count * 8), kScanThreads, s, p->edge_rec[pipe],
                        fanout, p->tile_state[pipe], p->ids[pipe], p->map[pipe], p->src_global[pipe], p->agg_src[pipe],
                        p->agg_dst[pipe], p->ctl[pipe], p->node_counter[pipe], p->edge_counter[pipe], op_id, p->bctl[pipe],
-                       hop + 1 == p->hop_num ? 1 : 0, p->max_nodes, p->max_edges, part));
+                       hop + 1 == p->hop_num ? 1 : 0, p->max_nodes, p->max_edges, part, g_scan_wait_limit));
     return LEGION_OK;
 }
 

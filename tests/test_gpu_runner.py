@@ -922,3 +922,40 @@ def test_host_table_packed_by_rank_serves_the_same_batches(oracle_mod, tmp_path)
     st = cache.stats()
     assert st["local_hits"] > 0 and st["misses"] > 0 and r.staged_rows() > 0
     r.Finalize(); pool.close(); cache.close(); fs.close(); g.close(); ds.close()
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_batch_that_an_error_ended_reports_its_own_sizes(oracle_mod, use_graph):
+    """Error 6 in the first hop, in the graph and launch by launch: the counters that collect_host returns, and the
+    page-locked mirror behind them, are those of the batch's seeds and not of the batch before on the pipe."""
+    batch = 1200
+    w = _world(oracle_mod, n=30000, pairs=300000, feat_len=16, batch=batch, cached_frac=0.3, seed=71)
+    nc, ec = np.zeros(16, np.int32), np.zeros(16, np.int32)
+
+    def one(r, gb):
+        r.submit_host(w["train"][:batch], w["labels"][:batch], gb)
+        return r.collect_host(None, None, None, None, nc, ec)
+
+    r = L.Runner(0, w["g"], w["f"], w["cache"], w["pool"], None)
+    r.set_options(use_graph=use_graph)
+    for gb in range(2):  # both pipes have held a whole batch
+        ref = oracle_mod.run_batch(w["indptr"], w["indices"], w["train"], w["labels"], batch, 0, w["fanout"], gb, 99)
+        assert one(r, gb) == (len(ref["ids"]), len(ref["agg_src"]))
+    r.Finalize()
+    L._check(L.lib().legion_set_tunable(b"scan_wait_limit", -1))
+    try:
+        r = L.Runner(0, w["g"], w["f"], w["cache"], w["pool"], None)
+        r.set_options(use_graph=use_graph)
+        for gb in range(2):
+            assert one(r, gb) == (batch, 0)
+            assert nc[9] == batch and nc[11] == batch and nc[3] == 0 and ec[10:12].sum() == 0
+        assert w["pool"].device_error(reset=True) == 6
+        r.Finalize()
+    finally:
+        L._check(L.lib().legion_set_tunable(b"scan_wait_limit", 1 << 20))
+    r = L.Runner(0, w["g"], w["f"], w["cache"], w["pool"], None)
+    r.set_options(use_graph=use_graph)
+    for gb in range(2):
+        assert one(r, gb) == (len(oracle_mod.run_batch(w["indptr"], w["indices"], w["train"], w["labels"], batch, 0, w["fanout"], gb, 99)["ids"]), ec[10:12].sum())
+    assert w["pool"].device_error() == 0
+    r.Finalize()

@@ -355,3 +355,79 @@ def test_sampling_ops_in_any_order(oracle_mod, fanout, ops, pipes):
     _run_ops(g, f, pool, batch, 0, fanout, global_batch=9)
     _compare(_fetch(pool), oracle_mod.run_batch(indptr, indices, train, train, batch, 0, fanout, 9, 21))
     pool.close(); f.close(); g.close()
+
+
+def _defined(got, ref_ids, fanout, limit_nodes):
+    """A batch that an error ended: counters of whole hops, indices in range, ids those of the replay."""
+    nc, ec = got["node_counter"], got["edge_counter"]
+    n, e = int(nc[0] + nc[1]), int(ec[0] + ec[1])
+    hops = len(fanout)
+    assert nc[8] == hops and nc[9] <= n <= limit_nodes and nc[9 + hops] == n and nc[6] == 0 and ec[2] == 0
+    np.testing.assert_array_equal(got["ids"], ref_ids[:n])
+    if e:
+        assert 0 <= got["agg_src"].min() and got["agg_src"].max() < n and 0 <= got["agg_dst"].min() and got["agg_dst"].max() < n
+    return n, e
+
+
+@pytest.mark.parametrize("pipes", [1, 2])
+def test_hop_that_does_not_fit_leaves_the_counters_of_the_hops_before(oracle_mod, pipes):
+    """The first hop twice over a dense graph has more edges than the pool: error 2 in the scan.  The batch stands as after
+    the first op, the ops behind it do nothing, and after the reset the pool works as before."""
+    fanout, batch, n_nodes = [20, 2], 64, 20000
+    indptr, indices = small_graph(n_nodes, 600000, 61)
+    train = np.random.default_rng(4).permutation(n_nodes)[:batch * 2].astype(np.int32)
+    g, f, pool = _setup(indptr, indices, train, train.copy(), batch, fanout, pipes=pipes)
+    pool.set_rng(3, 64)
+    for rep in range(2):
+        pool.set_batch(0, L.TRAINMODE, 0, rep)
+        L.BatchGenerate(None, f, None, pool, batch, 0, 0, 0, L.TRAINMODE, False, len(fanout))
+        for op in (3, 3, 6):
+            L.RandomSample(None, g, None, pool, fanout[op // 3 - 1], 0, op)
+        want = _replay_ops(oracle_mod, indptr, indices, train[:batch], fanout, [3], rep, 3)
+        full = _replay_ops(oracle_mod, indptr, indices, train[:batch], fanout, [3, 3], rep, 3)
+        assert len(full["agg_src"]) > pool.max_edges > len(want["agg_src"])
+        got = _fetch_known(pool)
+        n, e = _defined(got, want["ids"], fanout, len(want["ids"]))
+        assert (n, e) == (len(want["ids"]), len(want["agg_src"]))
+        np.testing.assert_array_equal(got["agg_src"], want["agg_src"])
+        np.testing.assert_array_equal(got["agg_dst"], want["agg_dst"])
+        assert pool.device_error(reset=True) == 2
+        _run_ops(g, f, pool, batch, 1, fanout, global_batch=rep)
+        _compare(_fetch(pool), oracle_mod.run_batch(indptr, indices, train, train, batch, 1, fanout, rep, 3))
+        assert pool.device_error() == 0
+    pool.close(); f.close(); g.close()
+
+
+@pytest.mark.parametrize("limit", [-1, 0])
+@pytest.mark.parametrize("pipes", [1, 2])
+def test_waits_of_the_scan_that_give_up(oracle_mod, limit, pipes):
+    """Waits that give up at once (-1), or after one read (0: some do, some do not).  The kernels return, error 6 is
+    reported, the counters are those of whole hops, no index is out of range, and the next batch is the replay's."""
+    fanout, batch, n_nodes = [25, 10], 4000, 60000
+    indptr, indices = small_graph(n_nodes, 700000, 62)
+    train = np.random.default_rng(6).permutation(n_nodes)[:batch].astype(np.int32)
+    g, f, pool = _setup(indptr, indices, train, train.copy(), batch, fanout, pipes=pipes)
+    pool.set_rng(8, 64)
+    errors = 0
+    for rep in range(6):
+        ref = oracle_mod.run_batch(indptr, indices, train, train, batch, 0, fanout, rep, 8)
+        L._check(L.lib().legion_set_tunable(b"scan_wait_limit", limit))
+        try:
+            _run_ops(g, f, pool, batch, 0, fanout, global_batch=rep, pipe=rep % pipes)
+        finally:
+            L._check(L.lib().legion_set_tunable(b"scan_wait_limit", 1 << 20))
+        got = _fetch_known(pool, rep % pipes)
+        n, e = _defined(got, ref["ids"], fanout, len(ref["ids"]))
+        assert got["edge_counter"][10:12].sum() == e
+        err = pool.device_error(reset=True)
+        assert err in (0, 6)
+        errors += err == 6
+        assert (n, e) in [(batch, 0)] if limit < 0 else (n, e) in [(batch, 0), (int(ref["node_counter"][10]), int(ref["edge_counter"][10])),
+                                                                   (len(ref["ids"]), len(ref["agg_src"]))]
+        if err == 0:
+            _compare(_fetch(pool, rep % pipes), ref)
+        _run_ops(g, f, pool, batch, 0, fanout, global_batch=rep, pipe=rep % pipes)
+        _compare(_fetch(pool, rep % pipes), ref)
+        assert pool.device_error() == 0
+    assert errors == 6 if limit < 0 else errors > 0
+    pool.close(); f.close(); g.close()
