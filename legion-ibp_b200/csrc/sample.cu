@@ -39,21 +39,23 @@ __device__ __forceinline__ uint32_t mix32(uint32_t h)
 }
 
 // One probe of map slot `m` for `key`.  True: the slot is the key's, and its value is at most `cand`.
-// A slot is read and claimed as one 8-byte word, key and value together: a key that is met for the first time
-// costs one load and one compare-and-swap, a key whose value is already below `cand` (a seed, a node of an
-// earlier hop, a hub that other inputs have reached) one load.  Values only fall and keys never change once
-// written, so a stale read can only lead to an atomic that changes nothing.
+// A slot is read, claimed and lowered as one 8-byte word, the value in its upper half, so that its accesses never
+// overlap in part: a key that is met for the first time costs one load and one compare-and-swap, a key whose value is
+// already below `cand` (a seed, a node of an earlier hop, a hub that other inputs have reached) one load.  Values (never
+// negative) only fall and keys never change once written, so a stale read can only lead to an atomic that changes
+// nothing.
 __device__ __forceinline__ bool map_claim(MapSlot *m, int32_t key, int32_t cand)
 {
     const unsigned long long empty = ((unsigned long long)(uint32_t)kEmptyVal << 32) | (uint32_t)kEmptyKey;
-    unsigned long long w = __ldcg(reinterpret_cast<const unsigned long long *>(m));
+    const unsigned long long mine = ((unsigned long long)(uint32_t)cand << 32) | (uint32_t)key;
+    unsigned long long *const word = reinterpret_cast<unsigned long long *>(m);
+    unsigned long long w = __ldcg(word);
     if (w == empty) {
-        w = atomicCAS(reinterpret_cast<unsigned long long *>(m), empty,
-                      ((unsigned long long)(uint32_t)cand << 32) | (uint32_t)key);
+        w = atomicCAS(word, empty, mine);
         if (w == empty) return true;
     }
     if ((int32_t)(uint32_t)w != key) return false;
-    if ((int32_t)(w >> 32) > cand) atomicMin(&m->val, cand);
+    if (w > mine) atomicMin(word, mine);
     return true;
 }
 
