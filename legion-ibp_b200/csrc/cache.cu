@@ -707,6 +707,7 @@ extern "C" int legion_cache_lut(LegionCache *c, int32_t **lut_dev)
     LG_ARG(c->part[c->kg] == nullptr, "the lookup table of a cache with replicas is only usable through the cache handle");
     LG_ARG(c->codec == LEGION_CODEC_RAW, "the lookup table of a compressed cache is only usable through the cache handle");
     *lut_dev = c->lut;
+    c->lut_given = 1;  // from now on what the table holds is not known
     return LEGION_OK;
 }
 

@@ -155,7 +155,8 @@ struct LegionCache {
     int32_t replica_rows;              // rows of part[kg] (legion_cache_add_replicas)
     int32_t fill_by_caller;            // set while legion_cache_place_static builds the table without copying rows
     int64_t fill_gen;                  // counts the changes of the lookup table (fill, replicas)
-    int32_t holds_all;                 // every node has a row in this GPU's own partition: no lookup can miss
+    int32_t holds_all;                 // every node has a row in this GPU's own partition when the table is filled
+    int32_t lut_given;                 // the caller has the table's address (legion_cache_lut) and may change entries
     legion::VmmBlock own_block;        // set when part[ki] is shareable memory (clique of more than one GPU)
     legion::VmmBlock peer_block[LEGION_MAX_DEVICE];  // partitions mapped from other processes
     // lru

@@ -1274,11 +1274,11 @@ int g_miss_threads = 0;  // 0 = default
 int g_miss_rows = 0;     // rows a warp of the fetch keeps in flight (0 = default, 4)
 
 // The rows the hit kernels listed so far, fetched from the pinned host table; empties the list.
-// No-op when nothing can be on the list: without a host table, or when the cache holds every node (the launch alone, over
-// an empty list, was 3 us of a batch).
+// No-op when nothing can be on the list: without a host table, or when the cache holds every node and only this library
+// has written its table (the launch alone, over an empty list, was 3 us of a batch).
 bool cache_may_miss(const LegionCache *c)
 {
-    return c != nullptr && c->host_table != nullptr && !c->holds_all;
+    return c != nullptr && c->host_table != nullptr && (!c->holds_all || c->lut_given);
 }
 
 int launch_gather_misses(cudaStream_t s, LegionPool *p, LegionCache *c)

@@ -139,3 +139,25 @@ def test_cache_that_holds_every_node_needs_no_fetch(oracle_mod):
         rig.cache.fill_static(torch.from_numpy(order[:10].copy()).cuda(), rig.h_table)
         np.testing.assert_array_equal(rig.gather(0)[1], table[ids])
         rig.close()
+
+
+def test_changed_table_of_a_cache_that_holds_every_node(oracle_mod):
+    """The caller takes the address of the lookup table of a full cache and marks nodes as missed: their rows come from the
+    host table again, call after call, and every call empties its list of them."""
+    import torch
+    rng = np.random.default_rng(9)
+    n, row_bytes, count = 600, 64, 600
+    table = rng.integers(0, 256, (n, row_bytes)).astype(np.uint8)
+    ids = rng.permutation(n).astype(np.int32)
+    rig = Rig(table, ids, count, capacity=n, order=rng.permutation(n).astype(np.int32))
+    np.testing.assert_array_equal(rig.gather(0)[1], table[ids])
+    lut = rig.cache.lut_ptr()
+    missed = np.full(n // 2, -2, np.int32)  # the first half of the nodes
+    L._check(L.lib().legion_copy(L.C.c_void_p(lut), missed.ctypes.data_as(L.C.c_void_p), L.C.c_int64(missed.nbytes), L.C.c_int32(1)))
+    rig.h_table[: n // 2] ^= 0x5A  # the host's rows are told from the cached ones
+    want = np.where((ids < n // 2)[:, None], table[ids] ^ 0x5A, table[ids])
+    for _ in range(8):  # more misses in all than the list has places
+        np.testing.assert_array_equal(rig.gather(0)[1], want)
+    st = rig.cache.stats()
+    assert st["misses"] == 8 * (n // 2) and st["local_hits"] == count + 8 * (n // 2)
+    rig.close()
