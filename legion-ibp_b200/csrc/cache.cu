@@ -330,7 +330,7 @@ extern "C" int legion_cache_create(LegionCache **out, int32_t dev_id, int64_t n_
         else
             e = cudaMalloc(&c->part[ki], (int64_t)capacity * c->slot_bytes);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&c->stats, sizeof(unsigned long long) * 4);
+    if (e == cudaSuccess) e = cudaMalloc(&c->stats, sizeof(unsigned long long) * 5);
     if (e != cudaSuccess) {
         set_error("legion_cache_create: cudaMalloc failed: %s", cudaGetErrorString(e));
         cudaFree(c->lut); cudaFree(c->stats);
@@ -427,21 +427,17 @@ __global__ void count_missing_kernel(const int32_t *__restrict__ lut, int64_t n,
     if (bad != 0) atomicAdd(missing, bad);
 }
 
-// Sets holds_all from the table just built.  Only a clique of one whose capacity covers the nodes is looked at.
+// Sets holds_all from the table just built.  Only a clique of one whose capacity covers the nodes is looked at.  (No
+// allocation: a cache may have been sized to fill the GPU.)
 static int find_holds_all(LegionCache *c, int64_t n_cached, int sms, cudaStream_t s)
 {
     if (c->kg != 1 || n_cached < c->n_nodes) return LEGION_OK;
-    int32_t *d = nullptr, missing = 1;
-    LG_CUDA(cudaMalloc(&d, sizeof(*d)));
-    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(*d), s);
-    if (e == cudaSuccess) {
-        count_missing_kernel<<<grid_stride(c->n_nodes, sms), 256, 0, s>>>(c->lut, c->n_nodes, c->capacity, d);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&missing, d, sizeof(missing), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d);
-    LG_CUDA(e);
+    int32_t *d = reinterpret_cast<int32_t *>(c->stats + 4), missing = 1;
+    LG_CUDA(cudaMemsetAsync(d, 0, sizeof(*d), s));
+    count_missing_kernel<<<grid_stride(c->n_nodes, sms), 256, 0, s>>>(c->lut, c->n_nodes, c->capacity, d);
+    LG_LAUNCH_CHECK();
+    LG_CUDA(cudaMemcpyAsync(&missing, d, sizeof(missing), cudaMemcpyDeviceToHost, s));
+    LG_CUDA(cudaStreamSynchronize(s));
     c->holds_all = missing == 0 ? 1 : 0;
     return LEGION_OK;
 }

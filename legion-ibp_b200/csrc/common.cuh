@@ -168,7 +168,7 @@ struct LegionCache {
     int32_t clock;
     const void *host_table;
     int32_t host_codec;         // codec of the host table's rows (RAW unless legion_cache_set_host_codec)
-    unsigned long long *stats;  // 4 counters on the device
+    unsigned long long *stats;  // 4 counters on the device; static caches: and a word for find_holds_all
 };
 
 namespace legion {

@@ -91,3 +91,48 @@ def test_rejects_lists_above_the_built_in_scratch():
                                             None, 0, 1, 0, None, None, C.c_int64(10), 16, C.c_void_p(out.data_ptr()))
     assert rc == -4
     assert b"above the built-in scratch" in L.lib().legion_last_error()
+
+
+def test_fill_of_a_full_cache_allocates_nothing(oracle_mod):
+    """A cache may have been sized to fill the GPU: with every byte of device memory taken, filling it with every node
+    still works."""
+    import torch
+    from cuda.bindings import runtime as rt
+    rng = np.random.default_rng(3)
+    n, row_bytes = 3000, 64
+    table = rng.integers(0, 256, (n, row_bytes)).astype(np.uint8)
+    h_table = torch.from_numpy(table).pin_memory()
+    order = torch.from_numpy(rng.permutation(n).astype(np.int32)).cuda()
+    ids_np = rng.permutation(n).astype(np.int32)
+    ids, lab = torch.from_numpy(ids_np).cuda(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    f = L.FeatureStorage(0, n, row_bytes, h_table)
+    f.set_split(L.TRAINMODE, ids, lab)
+    cache = L.UnifiedCache(0, n, row_bytes, n)
+    pool = L.MemoryPool(0, n, [], row_bytes, 1)
+
+    def rows():
+        pool.set_batch(0, L.TRAINMODE, 0, 0)
+        L.BatchGenerate(None, f, cache, pool, n, 0, 0, 0, L.TRAINMODE, False, 0)
+        L.FeatureCacheLookup(None, cache, pool, 1, 0)
+        return pool.read(L.BUF_FEATURES, 0, n * row_bytes, np.uint8).reshape(n, row_bytes)
+
+    cache.fill_static(order, h_table)   # the driver loads the kernels' code
+    np.testing.assert_array_equal(rows(), table[ids_np])
+    torch.cuda.synchronize()
+    taken = []
+    try:
+        size = torch.cuda.mem_get_info()[0]
+        while size >= 256:
+            err, p = rt.cudaMalloc(size)
+            if int(err) == 0:
+                taken.append(p)
+            else:
+                rt.cudaGetLastError()
+                size //= 2
+        cache.fill_static(order, h_table)
+    finally:
+        for p in taken:
+            rt.cudaFree(p)
+    np.testing.assert_array_equal(rows(), table[ids_np])
+    assert cache.stats()["misses"] == 0
+    pool.close(); cache.close(); f.close()
