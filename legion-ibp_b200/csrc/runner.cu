@@ -70,6 +70,8 @@ struct LegionRunner {
     cudaEvent_t hit_done[LEGION_MAX_PIPES];   // lookup + gather of the pipe's batch is over
     cudaEvent_t pipe_done[LEGION_MAX_PIPES];
     bool pipe_busy[LEGION_MAX_PIPES];
+    long long issued, pipe_issue[LEGION_MAX_PIPES];  // batches issued; number of the pipe's newest one ...
+    bool awaited[LEGION_MAX_PIPES];                  // ... which the host has waited for
     int current_pipe, last_pipe;
     bool use_graph, time_kernels;
     PipeGraph pg[LEGION_MAX_PIPES];
@@ -158,6 +160,18 @@ static const int32_t *final_counters(LegionRunner *r, int pipe)
     return hc;
 }
 
+// Waits for the batch on `pipe` and for every batch issued before it, which may end on a stream of its own.
+static cudaError_t wait_batch(LegionRunner *r, int pipe)
+{
+    for (int i = 0; i < LEGION_MAX_PIPES; ++i) {
+        if (r->awaited[i] || r->pipe_issue[i] > r->pipe_issue[pipe]) continue;
+        const cudaError_t e = cudaEventSynchronize(r->pipe_done[i]);
+        if (e != cudaSuccess) return e;
+        r->awaited[i] = true;
+    }
+    return cudaSuccess;
+}
+
 // The finished batch of `pipe` goes to the consumer: counters into the host segment, then the post.
 static int post_batch(LegionRunner *r, int pipe)
 {
@@ -197,6 +211,11 @@ extern "C" int legion_runner_create(LegionRunner **out, int32_t dev_id, LegionGr
     r->env = env;
     r->current_pipe = 0;
     r->last_pipe = -1;
+    r->issued = 0;
+    for (int i = 0; i < LEGION_MAX_PIPES; ++i) {
+        r->pipe_issue[i] = 0;
+        r->awaited[i] = true;
+    }
     r->use_graph = true;
     r->time_kernels = false;
     r->open_window = false;
@@ -564,6 +583,8 @@ static int issue_rest(LegionRunner *r, int pipe, int32_t host_seeds, bool bound,
     }
     if (lru) c->clock += 1;
     r->pipe_busy[pipe] = true;
+    r->pipe_issue[pipe] = ++r->issued;
+    r->awaited[pipe] = false;
     r->last_pipe = pipe;
     r->window_batches += 1;
     return LEGION_OK;
@@ -906,7 +927,7 @@ static int collect_host_body(LegionRunner *r, int32_t *ids_out, int32_t *labels_
     r->host_pending -= 1;
     {
         const double w0 = now_us();
-        LG_CUDA(cudaEventSynchronize(r->pipe_done[pipe]));
+        LG_CUDA(wait_batch(r, pipe));
         r->host_us[2] += now_us() - w0;
     }
     const int32_t *hc = (bound && p->hop_num > 0) ? kept : final_counters(r, pipe);
@@ -1010,6 +1031,7 @@ extern "C" int legion_runner_sync(LegionRunner *r)
     }
     for (int i = 0; i < LEGION_MAX_PIPES; ++i) {
         r->pipe_busy[i] = false;
+        r->awaited[i] = true;
         r->slot_busy[i] = false;
         r->pg[i].launched = false;
     }
@@ -1055,7 +1077,7 @@ extern "C" int legion_runner_run_once(LegionRunner *r, int32_t global_batch_id, 
     clock_gettime(CLOCK_MONOTONIC, &t0);
     int rc = legion_runner_enqueue(r, global_batch_id, mode, local_batch_id);
     if (rc != LEGION_OK) return rc;
-    LG_CUDA(cudaEventSynchronize(r->pipe_done[pipe]));  // engine/server.cu:356-361
+    LG_CUDA(wait_batch(r, pipe));  // engine/server.cu:356-361
     clock_gettime(CLOCK_MONOTONIC, &t1);
     r->served_us += (t1.tv_sec - t0.tv_sec) * 1e6 + (t1.tv_nsec - t0.tv_nsec) * 1e-3;
     r->served += 1;
@@ -1103,14 +1125,14 @@ extern "C" int legion_runner_serve(LegionRunner *r, int32_t first_global_batch, 
             rc = issue_rest(r, pipe, 0, false, false);
             if (rc != LEGION_OK) return rc;
             if (prev_pipe >= 0) {
-                LG_CUDA(cudaEventSynchronize(r->pipe_done[prev_pipe]));
+                LG_CUDA(wait_batch(r, prev_pipe));
                 rc = post_batch(r, prev_pipe);
                 if (rc != LEGION_OK) return rc;
             }
             prev_pipe = pipe;
         }
         if (prev_pipe >= 0) {
-            LG_CUDA(cudaEventSynchronize(r->pipe_done[prev_pipe]));
+            LG_CUDA(wait_batch(r, prev_pipe));
             int rc = post_batch(r, prev_pipe);
             if (rc != LEGION_OK) return rc;
         }
@@ -1123,14 +1145,14 @@ extern "C" int legion_runner_serve(LegionRunner *r, int32_t first_global_batch, 
         rc = legion_runner_enqueue(r, b, legion_ipc_current_mode(r->env, b), legion_ipc_local_batch_id(r->env, b));
         if (rc != LEGION_OK) return rc;
         if (prev_pipe >= 0) {
-            LG_CUDA(cudaEventSynchronize(r->pipe_done[prev_pipe]));
+            LG_CUDA(wait_batch(r, prev_pipe));
             rc = post_batch(r, prev_pipe);
             if (rc != LEGION_OK) return rc;
         }
         prev_pipe = pipe;
     }
     if (prev_pipe >= 0) {
-        LG_CUDA(cudaEventSynchronize(r->pipe_done[prev_pipe]));
+        LG_CUDA(wait_batch(r, prev_pipe));
         int rc = post_batch(r, prev_pipe);
         if (rc != LEGION_OK) return rc;
     }

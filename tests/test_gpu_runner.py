@@ -959,3 +959,42 @@ def test_batch_that_an_error_ended_reports_its_own_sizes(oracle_mod, use_graph):
         assert one(r, gb) == (len(oracle_mod.run_batch(w["indptr"], w["indices"], w["train"], w["labels"], batch, 0, w["fanout"], gb, 99)["ids"]), ec[10:12].sum())
     assert w["pool"].device_error() == 0
     r.Finalize()
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_run_once_returns_behind_the_batches_enqueued_before(oracle_mod, use_graph):
+    """With every node cached a batch ends on its pipe's own stream: a small batch must not be handed over while a large
+    one that was enqueued before it is still being gathered."""
+    import torch
+    rng = np.random.default_rng(12)
+    n, feat_len, batch = 100000, 512, 600000
+    h_table = torch.from_numpy(rng.standard_normal((n, feat_len)).astype(np.float32)).pin_memory()
+    train = np.concatenate([rng.integers(0, n, batch), [5, 6, 7]]).astype(np.int32)
+    d_train = torch.from_numpy(train).cuda()
+    d_indptr, d_indices = torch.zeros(n + 1, dtype=torch.int64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    g = L.GraphStorage(0, d_indptr, d_indices)
+    f = L.FeatureStorage(0, n, feat_len * 4, h_table)
+    f.set_split(L.TRAINMODE, d_train, d_train)
+    cache = L.UnifiedCache(0, n, feat_len * 4, n)
+    cache.fill_static(torch.arange(n, dtype=torch.int32, device="cuda"), h_table)
+    pool = L.MemoryPool(0, batch, [], feat_len * 4, 2)
+    r = L.Runner(0, g, f, cache, pool, None)
+    r.set_options(use_graph=use_graph)
+    r.enqueue(0, L.TRAINMODE, 1)
+    r.enqueue(1, L.TRAINMODE, 1)
+    r.sync()
+    rows, _ = pool.buffer(L.BUF_FEATURES, 0)
+    blank_row, got = np.full(feat_len, -1.0, np.float32), np.empty(feat_len, np.float32)
+    for rep in range(3):
+        # the last row of the large batch's buffer, before and right after
+        L._check(L.lib().legion_copy(L.C.c_void_p(rows + (batch - 1) * feat_len * 4), blank_row.ctypes.data_as(L.C.c_void_p),
+                                     L.C.c_int64(feat_len * 4), L.C.c_int32(1)))
+        r.enqueue(2 * rep, L.TRAINMODE, 0)
+        r.RunOnce(2 * rep + 1, L.TRAINMODE, 1)
+        L._check(L.lib().legion_copy(got.ctypes.data_as(L.C.c_void_p), L.C.c_void_p(rows + (batch - 1) * feat_len * 4),
+                                     L.C.c_int64(feat_len * 4), L.C.c_int32(2)))
+        np.testing.assert_array_equal(got, h_table[int(train[batch - 1])].numpy())
+        small = pool.read(L.BUF_FEATURES, 1, 3 * feat_len, np.float32).reshape(3, feat_len)
+        np.testing.assert_array_equal(small, h_table[5:8].numpy())
+    r.Finalize()
+    pool.close(); cache.close(); f.close(); g.close()
