@@ -72,8 +72,8 @@ int legion_set_tunable(const char *name, int32_t value);
  * "gather_rows_in_flight" (2/4/8/16, register path); "gather_engine" 0 = rows move through registers,
  * 1 = rows move by bulk asynchronous copies through shared memory (start value from the environment
  * variable LEGION_GATHER_ENGINE); "pdl" 1 = the sampling kernels of a batch are launched as programmatic
- * dependents of one another in every pool (start value from LEGION_PDL; applies to runners created afterwards), 0 = only
- * in pools of one pipe or at most 65,536 nodes;
+ * dependents of one another, 0 = they are not, -1 (the default) = in pools of one pipe or at most 65,536 nodes (start
+ * value from LEGION_PDL; applies to ops issued and runners created afterwards);
  * "scan_wait_limit": reads of a wait inside the scan of a hop before it gives up (default 2^20, about a second; 0 and, for
  * waits that give up whatever they read, -1 are for tests; applies to ops issued and runners created afterwards);
  * "map_front_shift" s: the front region of a pool's id map gets 1 / 2^s of the worst-case slots

@@ -1512,7 +1512,7 @@ extern "C" int legion_set_tunable(const char *name, int32_t value)
         return LEGION_OK;
     }
     if (strcmp(name, "pdl") == 0) {
-        LG_ARG(value == 0 || value == 1, "pdl must be 0 or 1");
+        LG_ARG(value >= -1 && value <= 1, "pdl must be -1 (by the pool), 0 or 1");
         g_pdl = value;  // takes effect for runners created (graphs captured) afterwards
         return LEGION_OK;
     }

@@ -27,7 +27,7 @@ static constexpr unsigned kFull = 0xFFFFFFFFu;
 // predecessor in the stream is still running; it must not touch the predecessor's results before
 // pdl_wait() returns (all prerequisite grids complete, their writes visible).  pdl_trigger() lets the
 // successor of THIS kernel be scheduled as soon as every CTA of this kernel has started.  Both are
-// no-ops for a kernel launched the ordinary way.  The point: a hop is four 8-20 us kernels, and the
+// no-ops for a kernel launched the ordinary way.  The point: a hop is two kernels of 5-25 us, and the
 // drain / launch / ramp-up between two of them costs as much as a quarter of one.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -548,12 +548,13 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
 
 // ---- launchers -----------------------------------------------------------------------------------
 
-// 1: the kernels of a batch after its first are launched as programmatic dependents (legion_set_tunable
-// "pdl"; start value from the environment variable LEGION_PDL)
+// 1: the kernels of a batch after its first are launched as programmatic dependents; 0: never; -1: by the rule below
+// (legion_set_tunable "pdl"; start value from the environment variable LEGION_PDL)
 static int pdl_from_env()
 {
     const char *v = getenv("LEGION_PDL");
-    return (v != nullptr && v[0] == '1' && v[1] == 0) ? 1 : 0;
+    if (v == nullptr || (v[0] != '0' && v[0] != '1') || v[1] != 0) return -1;
+    return v[0] - '0';
 }
 int g_pdl = pdl_from_env();
 // front region of the id map = worst-case slots >> this; -1: sized by legion_pool_create's own rule
@@ -577,7 +578,7 @@ static cudaError_t launch_dep(const LegionPool *p, void (*kernel)(KArgs...), int
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
-    const bool dependent = g_pdl || p->pipes == 1 || p->max_nodes <= kDependentNodes;
+    const bool dependent = g_pdl < 0 ? p->pipes == 1 || p->max_nodes <= kDependentNodes : g_pdl == 1;
     cfg.attrs = dependent ? at : nullptr;
     cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);

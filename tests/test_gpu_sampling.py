@@ -431,3 +431,24 @@ def test_waits_of_the_scan_that_give_up(oracle_mod, limit, pipes):
         assert pool.device_error() == 0
     assert errors == 6 if limit < 0 else errors > 0
     pool.close(); f.close(); g.close()
+
+
+@pytest.mark.parametrize("pdl", [0, 1])
+@pytest.mark.parametrize("n_nodes,n_pairs,batch,fanout,pipes", [(3000, 40000, 200, [5, 5, 5], 1), (3000, 40000, 200, [5, 5, 5], 2),
+                                                                (500, 20000, 50, [32, 32], 1), (150000, 4000000, 9000, [25, 16], 1),
+                                                                (150000, 4000000, 9000, [25, 16], 2)])
+def test_dependent_and_ordinary_launches(oracle_mod, pdl, n_nodes, n_pairs, batch, fanout, pipes):
+    """Both ways of launching the kernels of a hop, small hops and hops of more CTAs than run at once, one pipe and two."""
+    indptr, indices = small_graph(n_nodes, n_pairs, 81)
+    train = np.random.default_rng(5).permutation(n_nodes)[:batch].astype(np.int32)
+    g, f, pool = _setup(indptr, indices, train, train.copy(), batch, fanout, pipes=pipes)
+    pool.set_rng(17, 64)
+    L._check(L.lib().legion_set_tunable(b"pdl", pdl))
+    try:
+        for it in range(3):
+            _run_ops(g, f, pool, batch, 0, fanout, global_batch=it, pipe=it % pipes)
+            _compare(_fetch(pool, it % pipes), oracle_mod.run_batch(indptr, indices, train, train, batch, 0, fanout, it, 17))
+            assert pool.device_error() == 0
+    finally:
+        L._check(L.lib().legion_set_tunable(b"pdl", -1))
+    pool.close(); f.close(); g.close()
