@@ -161,3 +161,38 @@ def test_changed_table_of_a_cache_that_holds_every_node(oracle_mod):
     st = rig.cache.stats()
     assert st["misses"] == 8 * (n // 2) and st["local_hits"] == count + 8 * (n // 2)
     rig.close()
+
+
+@pytest.mark.parametrize("codec", [L.CODEC_INT8, L.CODEC_E4M3])
+@pytest.mark.parametrize("feat_len", [4, 60, 128, 132, 516, 772, 1028, 2052])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_encoder_rows_with_infinities_and_nan(oracle_mod, codec, feat_len, shift):
+    """Rows that are not all finite, in the lanes' registers and behind them, beside rows that are: an infinity makes the
+    scale infinite and every finite code 0, a NaN leaves the scale to the other values and is stored as 0 (int8) or
+    0x7F (e4m3; the host may write its sign)."""
+    import torch
+    rng = np.random.default_rng(feat_len)
+    n = 41
+    x = rng.standard_normal((n, feat_len)).astype(np.float32)
+    last = feat_len - 1
+    x[0, 0] = np.inf
+    x[3, last] = -np.inf
+    x[4, last] = np.nan
+    x[7, 0] = -np.nan
+    x[8] = np.nan
+    x[9] = np.inf
+    x[12, 0], x[12, last] = np.nan, np.inf
+    x[13] = 0.0
+    x[13, last] = np.nan
+    x[20, rng.integers(0, feat_len)] = np.inf
+    x[21, rng.integers(0, feat_len)] = np.nan
+    x[n - 1, last] = np.nan
+    src = torch.zeros(n * feat_len + 1, device="cuda")
+    src[shift:shift + n * feat_len] = torch.from_numpy(x).reshape(-1).cuda()
+    out = torch.full((n, oracle_mod.quant_row_bytes(feat_len)), 7, dtype=torch.uint8, device="cuda")
+    L.quantize_table(0, codec, src[shift:], n, feat_len, out)
+    with np.errstate(invalid="ignore"):
+        want = oracle_mod.quant_rows(x, codec)
+    if codec == L.CODEC_E4M3:
+        want[:, :feat_len] = np.where(want[:, :feat_len] == 0xFF, 0x7F, want[:, :feat_len])
+    np.testing.assert_array_equal(out.cpu().numpy(), want)

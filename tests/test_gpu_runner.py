@@ -998,3 +998,114 @@ def test_run_once_returns_behind_the_batches_enqueued_before(oracle_mod, use_gra
         np.testing.assert_array_equal(small, h_table[5:8].numpy())
     r.Finalize()
     pool.close(); cache.close(); f.close(); g.close()
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_hand_off_sequences_with_every_node_cached(oracle_mod, use_graph, tmp_path, monkeypatch):
+    """The host-buffer calls, the batches sampled ahead and the hand-off to a trainer, with a cache that holds every node:
+    nothing is fetched, and a batch ends on its pipe's own stream."""
+    import functools
+    monkeypatch.setitem(globals(), "_world", functools.partial(_world, cached_frac=1.0))
+    test_submit_collect_host_pipelined(oracle_mod, use_graph)
+    test_submit_host_to_writes_pinned_buffers(oracle_mod, use_graph)
+    test_batches_sampled_ahead_of_two_handoff_slots(oracle_mod, use_graph)
+    test_client_api_consumes_batches(oracle_mod, tmp_path, 4 if use_graph else 2)
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("pipes,slots", [(2, None), (4, None), (4, 2)])
+def test_runner_while_the_cache_goes_from_full_to_partial_and_back(oracle_mod, use_graph, pipes, slots):
+    """One runner over a cache that is filled with every node, then with a third of them, then with every node again:
+    batches end on their own stream, on the fetch stream, and on their own again, several pipes deep."""
+    w = _world(oracle_mod, seed=41, pipes=pipes, slots=slots, cached_frac=1.0)
+    held = slots or pipes
+    r = L.Runner(0, w["g"], w["f"], w["cache"], w["pool"], None)
+    r.set_options(use_graph=use_graph, time_kernels=True)
+    gb, misses = 0, []
+    for share in (1.0, 0.3, 1.0, 0.002, 1.0):
+        w["cache"].fill_static(w["d_order"][: int(w["n"] * share)].contiguous(), w["h_table"])
+        before = w["cache"].stats()["misses"]
+        for count in (1, pipes, 3 * pipes + 1):
+            first = gb
+            for _ in range(count):
+                r.enqueue(gb, L.TRAINMODE, gb % 6)
+                gb += 1
+            r.sync()
+            t = r.timing()
+            assert t["batches"] == t["timed"] == count and t["batch_ms"] >= t["gather_ms"] / count and (t["miss_ms"] > 0) == (share < 1.0)
+            for b in range(max(first, gb - held), gb):
+                _check_pipe(oracle_mod, w, (b % pipes) % held, b % 6, b)
+        r.RunOnce(gb, L.TRAINMODE, gb % 6)
+        _check_pipe(oracle_mod, w, (gb % pipes) % held, gb % 6, gb)
+        r.sync()
+        gb += 1
+        misses.append(w["cache"].stats()["misses"] - before)
+    assert [m > 0 for m in misses] == [False, True, False, True, False]
+    assert w["pool"].device_error() == 0
+    r.Finalize()
+
+
+HANDOFF = [(75, "raw", 0), (128, "raw", 0), (256, "raw", 0), (384, "raw", 0), (512, "raw", 0), (600, "raw", 0), (128, "raw", 1), (256, "raw", 1),
+           (75, "raw", 1), (100, "int8", 0), (100, "e4m3", 0), (200, "int8", 0), (300, "e4m3", 0), (128, "int8", 1)]
+
+
+@pytest.mark.parametrize("feat_len,codec,engine", HANDOFF)
+@pytest.mark.parametrize("cached_frac,host_codec", [(1.0, False), (0.3, False), (0.3, True)])
+def test_every_gather_hands_the_block_structure_over(oracle_mod, feat_len, codec, engine, cached_frac, host_codec):
+    """Batches sampled ahead, through each kernel that copies a block structure into its slot: rows of one to four vectors
+    a lane, rows that are no whole vectors, rows above 2048 bytes, decoded rows, and the bulk-copy engine."""
+    import torch
+    if host_codec and codec == "raw":
+        pytest.skip("a raw cache has no compressed host table")
+    w = _world(oracle_mod, n=4000, pairs=50000, feat_len=feat_len, batch=64, seed=feat_len, pipes=4, slots=2, cached_frac=cached_frac)
+    if codec != "raw":
+        which = {"int8": L.CODEC_INT8, "e4m3": L.CODEC_E4M3}[codec]
+        cap = int(w["n"] * cached_frac)
+        stored = oracle_mod.quant_rows(w["table"], which)
+        plain = oracle_mod.dequant_rows(stored, feat_len, which)
+        host = torch.from_numpy(stored).pin_memory() if host_codec else w["h_table"]
+        w["cache"] = L.UnifiedCache(0, w["n"], feat_len * 4, cap, codec=which)
+        if host_codec:
+            w["cache"].set_host_codec(which)
+        w["cache"].fill_static(w["d_order"], host)
+        cached = np.isin(np.arange(w["n"]), w["d_order"][:cap].cpu().numpy())
+        w["table"] = plain if host_codec else np.where(cached[:, None], plain, w["table"])
+    L._check(L.lib().legion_set_tunable(b"gather_engine", engine))
+    try:
+        r = L.Runner(0, w["g"], w["f"], w["cache"], w["pool"], None)
+        gb = 0
+        for count in (4, 1, 7, 2, 6):
+            for _ in range(count):
+                r.enqueue(gb, L.TRAINMODE, (5 * gb) % 7)   # the list's short last batch among them
+                gb += 1
+            r.sync()
+            for b in range(max(0, gb - 2), gb):
+                _check_pipe(oracle_mod, w, b % 2, (5 * b) % 7, b)
+        r.Finalize()
+    finally:
+        L._check(L.lib().legion_set_tunable(b"gather_engine", 0))
+    assert w["pool"].device_error() == 0
+
+
+@pytest.mark.parametrize("pdl", [-1, 0, 1])
+@pytest.mark.parametrize("pipes,batch,slots", [(2, 300, None), (4, 300, None), (4, 300, 2), (4, 96, 2)])
+def test_runner_graphs_of_ordinary_and_dependent_launches(oracle_mod, pdl, pipes, batch, slots):
+    """Captured sampling of pools above and below 65,536 nodes, launched both ways."""
+    w = _world(oracle_mod, n=20000, pairs=300000, feat_len=16, batch=batch, seed=53, pipes=pipes, slots=slots)
+    assert (w["pool"].max_nodes > 65536) == (batch == 300)
+    held = slots or pipes
+    L._check(L.lib().legion_set_tunable(b"pdl", pdl))
+    try:
+        r = L.Runner(0, w["g"], w["f"], w["cache"], w["pool"], None)
+        gb = 0
+        for count in (pipes, 1, 3 * pipes):
+            for _ in range(count):
+                r.enqueue(gb, L.TRAINMODE, gb % 7)
+                gb += 1
+            r.sync()
+            for b in range(max(0, gb - held), gb):
+                _check_pipe(oracle_mod, w, (b % pipes) % held, b % 7, b)
+        r.Finalize()
+    finally:
+        L._check(L.lib().legion_set_tunable(b"pdl", -1))
+    assert w["pool"].device_error() == 0
