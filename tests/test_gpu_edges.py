@@ -196,3 +196,33 @@ def test_encoder_rows_with_infinities_and_nan(oracle_mod, codec, feat_len, shift
     if codec == L.CODEC_E4M3:
         want[:, :feat_len] = np.where(want[:, :feat_len] == 0xFF, 0x7F, want[:, :feat_len])
     np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("batch", [300, 16383, 16384, 16385, 40000])
+@pytest.mark.parametrize("share", [0.0, 0.01, 1.0])
+def test_lru_lists_of_pools_that_order_them_and_that_do_not(oracle_mod, batch, share):
+    """Pools on both sides of the 16,384 rows at worst from which a list of missed rows is ordered, with lists that are
+    empty, short and as long as the batch: rows, hit / miss sets and counters follow the host replay."""
+    rng = np.random.default_rng(batch)
+    n, feat_len, sets, ways = 100000, 16, 12000, 8
+    table = rng.standard_normal((n, feat_len)).astype(np.float32)
+    nodes = rng.permutation(n)
+    first, cold = nodes[:batch], nodes[batch:2 * batch]
+    lists = [first]
+    missed = int(share * batch)
+    for _ in range(2):
+        lists.append(rng.permutation(np.concatenate([rng.permutation(first)[:batch - missed], rng.permutation(cold)[:missed]])))
+    flat = np.concatenate(lists).astype(np.int32)
+    rig = Rig(table, flat, batch, lru=(sets, ways))
+    ref = oracle_mod.LruCache(sets, ways)
+    for it in range(3):
+        ids, clock = flat[it * batch:(it + 1) * batch], rig.cache.lru_clock()
+        before = rig.cache.stats()["misses"]
+        cnt, feat, _ = rig.gather(it)
+        assert cnt == batch
+        ci = ref.lookup(ids, clock)
+        np.testing.assert_array_equal(rig.pool.read(L.BUF_CACHE_INDEX, 0, cnt, np.int64), ci)
+        np.testing.assert_array_equal(feat.view(np.float32).reshape(cnt, feat_len), table[ids])
+        assert rig.cache.stats()["misses"] - before == (ci < 0).sum()
+        ref.insert(ids, ci, clock)
+    rig.close()
