@@ -967,7 +967,7 @@ def test_run_once_returns_behind_the_batches_enqueued_before(oracle_mod, use_gra
     one that was enqueued before it is still being gathered."""
     import torch
     rng = np.random.default_rng(12)
-    n, feat_len, batch = 100000, 512, 600000
+    n, feat_len, batch = 100000, 128, 6000000  # 512-byte rows: the gather leaves room on the SMs for another batch
     h_table = torch.from_numpy(rng.standard_normal((n, feat_len)).astype(np.float32)).pin_memory()
     train = np.concatenate([rng.integers(0, n, batch), [5, 6, 7]]).astype(np.int32)
     d_train = torch.from_numpy(train).cuda()
