@@ -561,10 +561,11 @@ int g_pdl = pdl_from_env();
 // (legion_set_tunable "map_front_shift")
 int g_map_front_shift = -1;
 
-// Without the tunable, batches that have the GPU to themselves are launched this way too: pools of one pipe, and small
-// ones, whose launches are mostly start and drain.  Measured: 1,237 seeds,
-// [15,10], through the operators 115 -> 107 us, 32 seeds, [10,5], 80.5 -> 79.7; with four pipes of 800 seeds, [25,10], whose
-// kernels fill each other's gaps, nothing.
+// The rule: batches that have the GPU to themselves, in pools of one pipe, and small ones, whose launches are mostly start
+// and drain.  Measured, us a batch, ordinary against dependent launches, fanout [25,10], all rows cached: one pipe
+// 59.3 / 51.6 (pool of 65,494 nodes), 71.7 / 65.0 (228,800), 120 / 114 (2.3 M); two pipes 23.3 / 22.3, 29.6 / 29.1,
+// 64.2 / 66.3; four pipes 13.2 / 12.9, 18.6 / 18.7, 51.9 / 56.0, and at 128,700 nodes 15.3 / 15.1: with several pipes the
+// others' kernels fill the gaps, and the CTAs that wait take registers from them.
 constexpr int64_t kDependentNodes = 1 << 16;
 
 template <typename... KArgs, typename... Args>
