@@ -488,7 +488,7 @@ hop_finish_kernel(const int2 *__restrict__ rec, int32_t fanout, uint32_t *tile_s
 #pragma unroll
         for (int w = 0; w < kScanThreads / 32; ++w) { edges += s_edges[w]; fresh += s_new[w]; }
         const int tile_edges = tile_count & 0xFFFF, tile_new = tile_count >> 16;
-        // (cannot happen with the buffers that legion_pool_create sizes for this fanout)
+        // (in the pool's order they always fit: legion_pool_create sizes both buffers for it)
         if (failed == DERR_NONE && (int64_t)e_base + edges + tile_edges > max_edges) failed = DERR_EDGE_OVERFLOW;
         if (failed == DERR_NONE && (int64_t)n0 + fresh + tile_new > max_nodes) failed = DERR_NODE_OVERFLOW;
         if (failed != DERR_NONE && threadIdx.x == 0) atomicCAS(&ctl[CTL_LATE_ERROR], DERR_NONE, failed);
