@@ -226,3 +226,66 @@ def test_lru_lists_of_pools_that_order_them_and_that_do_not(oracle_mod, batch, s
         assert rig.cache.stats()["misses"] - before == (ci < 0).sum()
         ref.insert(ids, ci, clock)
     rig.close()
+
+
+@pytest.mark.parametrize("pipes", [1, 2])
+@pytest.mark.parametrize("kind", ["full", "part", "lru"])
+def test_operators_under_stream_capture(oracle_mod, pipes, kind):
+    """A caller captures a whole batch of operators, and an allocation-free gather behind it, in a graph of its own and
+    replays it over other seeds: ordinary and dependent launches, with and without a fetch."""
+    import torch
+    n, feat_len, batch, fanout = 6000, 32, 200, [25, 10]
+    indptr, indices = small_graph(n, 60000, 91)
+    rng = np.random.default_rng(14)
+    table = rng.standard_normal((n, feat_len)).astype(np.float32)
+    h_table = torch.from_numpy(table).pin_memory()
+    d_ip, d_ix = torch.from_numpy(indptr).cuda(), torch.from_numpy(indices).cuda()
+    g, f = L.GraphStorage(0, d_ip, d_ix), L.FeatureStorage(0, n, feat_len * 4, h_table)
+    seeds, labels = torch.zeros(batch, dtype=torch.int32, device="cuda"), torch.zeros(batch, dtype=torch.int32, device="cuda")
+    f.set_split(L.TRAINMODE, seeds, labels)
+    order = torch.from_numpy(rng.permutation(n).astype(np.int32)).cuda()
+    if kind == "lru":
+        cache = L.UnifiedCache(0, n, feat_len * 4, 0, lru=(100, 8))
+        cache.set_host_table(h_table)
+    else:
+        cache = L.UnifiedCache(0, n, feat_len * 4, n if kind == "full" else n // 4)
+        cache.fill_static(order, h_table)
+    plain = L.UnifiedCache(0, n, feat_len * 4, n // 4)
+    plain.fill_static(order, h_table)
+    lut, part = plain.lut_ptr(), [plain.partition()[0]]
+    rows = torch.zeros((batch, feat_len), device="cuda")
+    pool = L.MemoryPool(0, batch, fanout, feat_len * 4, pipes)
+    pool.set_rng(23, 64)
+    pool.set_batch(0, L.TRAINMODE, pipes - 1, 6)
+    stream = torch.cuda.Stream()
+
+    def ops():
+        L.run_batch(stream, g, f, cache, pool, 0)
+        L.gather_rows_noalloc(stream, 0, seeds, lut, n // 4, 1, 0, part, h_table, n, feat_len * 4, rows)
+
+    torch.cuda.synchronize()
+    ops()   # the driver loads the kernels' code
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        ops()
+    for rep in range(4):
+        train = rng.permutation(n)[:batch].astype(np.int32)
+        seeds.copy_(torch.from_numpy(train))
+        rows.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        ref = oracle_mod.run_batch(indptr, indices, train, np.zeros(batch, np.int32), batch, 0, fanout, 6, 23)
+        pipe = pipes - 1
+        np.testing.assert_array_equal(pool.read(L.BUF_NODE_COUNTER, pipe, 16, np.int32), ref["node_counter"])
+        np.testing.assert_array_equal(pool.read(L.BUF_EDGE_COUNTER, pipe, 16, np.int32), ref["edge_counter"])
+        np.testing.assert_array_equal(pool.read(L.BUF_IDS, pipe, len(ref["ids"]), np.int32), ref["ids"])
+        for which, key in ((L.BUF_AGG_SRC, "agg_src"), (L.BUF_AGG_DST, "agg_dst")):
+            np.testing.assert_array_equal(pool.read(which, pipe, len(ref[key]), np.int32), ref[key])
+        feat = pool.read(L.BUF_FEATURES, pipe, len(ref["ids"]) * feat_len, np.float32).reshape(-1, feat_len)
+        np.testing.assert_array_equal(feat, table[ref["ids"]])
+        np.testing.assert_array_equal(rows.cpu().numpy(), table[train])
+        assert pool.device_error() == 0
+    del graph
+    pool.close(); cache.close(); plain.close(); f.close(); g.close()
